@@ -165,6 +165,12 @@ GAS_HD double h_RT(const Tables &t, int k, double T) {
     const double *a = nasa(t, k, T);
     return a[0] + T * (a[1] / 2 + T * (a[2] / 3 + T * (a[3] / 4 + T * a[4] / 5))) + a[5] / T;
 }
+// h_RT with the polynomial's quotients a2/2 .. a5/5 formed once on the host (hcoef): one division
+// instead of three (a2/2 and a4/4 are exact), the last term's rounding apart the same value.
+GAS_HD double h_RT_q(const Tables &t, int k, double T) {
+    const double *c = t.hcoef[k][T < t.m.T_mid[k] ? 0 : 1];
+    return c[0] + T * (c[1] + T * (c[2] + T * (c[3] + T * c[4]))) + c[5] / T;
+}
 GAS_HD double s_R(const Tables &t, int k, double T) {
     const double *a = nasa(t, k, T);
     return a[0] * log(T) + T * (a[1] + T * (a[2] / 2 + T * (a[3] / 3 + T * a[4] / 4))) + a[6];
@@ -187,7 +193,7 @@ GAS_HD double cp_mass(const Tables &t, const double *Y, double T) {
 }
 GAS_HD double int_energy_mass(const Tables &t, const double *Y, double T) {
     double u = 0.0;
-    for (int k = 0; k < t.ns; ++k) u += Y[k] * (h_RT(t, k, T) - 1.0) * t.invW[k];
+    for (int k = 0; k < t.ns; ++k) u += Y[k] * (h_RT_q(t, k, T) - 1.0) * t.invW[k];
     return u * kR * T;
 }
 GAS_HD double cv_mass(const Tables &t, const double *Y, double T) {

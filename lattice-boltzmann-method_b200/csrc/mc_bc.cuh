@@ -2,7 +2,8 @@
 // free-slip, inflow or outflow cell upstream along some direction): streaming with the
 // reference's per-type rules, the Tamm-Mott-Smith boundary treatment (characteristic
 // outflow with NSCBC, characteristic inflow with the inline LODI relaxation, solid wall),
-// then the moments.  Host/device, like mc_cell.cuh.
+// then the moments.  Host/device, like mc_cell.cuh; the host build runs the whole cell
+// (mc_special_cell), the device the same operations by a block per 32 cells (mc_special.cuh).
 //
 // Reference path (farrasarira/Lattice-Boltzmann-Method, MULTICOMP on):
 //   LBM::Streaming                      src/lbm-streaming.cpp:3-119

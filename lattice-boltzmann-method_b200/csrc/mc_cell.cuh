@@ -1049,7 +1049,7 @@ MC_HDN void mc_eflux_cell(const AT &A, long n) {
     for (int a = 0; a < NS; ++a) {
         const double ha =
             fast ? u_energy_mass(A.U, (float)(gas::h_RT_fast(t, a, T_si, invT) * gas::kR * T_si * t.invW[a]))
-                 : u_energy_mass(A.U, (float)(gas::h_RT(t, a, T_si) * gas::kR * T_si / t.m.W[a]));
+                 : u_energy_mass(A.U, (float)(gas::h_RT_q(t, a, T_si) * gas::kR * T_si / t.m.W[a]));
         const int pr = rs(a, RS_RHO);
         const double rho_a = rec(A, Rc, pr, n);
         const double ua[3] = {rec(A, Rc, rs(a, RS_UX), n), rec(A, Rc, rs(a, RS_UX + 1), n),

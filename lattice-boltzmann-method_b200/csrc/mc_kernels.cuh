@@ -3,15 +3,14 @@
 // mc_ns<NS>.cu; the handle operations that dispatch to them are in mc.cu).
 //
 // Reference path replaced (farrasarira/Lattice-Boltzmann-Method, MULTICOMP on):
-//   LBM::Collide_Species + LBM::Collide   src/lbm-collision.cpp:191-526 -> k_mc_props, k_mc_chem (stiff
-//                                          chemistry or the surrogate's use; the surrogate's kernels,
-//                                          k_mc_chem_list), k_mc_eflux, k_mc_relax
+//   LBM::Collide_Species + LBM::Collide   src/lbm-collision.cpp:191-526 -> k_mc_props, the stiff
+//                                          chemistry (mc_chem.cuh), k_mc_eflux, k_mc_relax
 //   LBM::Streaming + LBM::calculate_moment src/lbm-streaming.cpp, src/lbm-moment.cpp:193-377
 //                                          -> k_mc_gather (pull + population sums per
 //                                             (cell, set)) and k_mc_solve (per cell)
 //   LBM::Init                              src/lbm-init.cpp:85-146 -> k_mc_init
 //   LBM::Streaming + LBM::TMS_BC + LBM::calculate_moment of the cells with a boundary
-//   upstream (src/lbm-bc.cpp:122-1110, src/impose_nscbc.cpp) -> k_mc_special
+//   upstream (src/lbm-bc.cpp:122-1110, src/impose_nscbc.cpp) -> k_mc_special (mc_special.cuh)
 #pragma once
 #include <algorithm>
 #include <cstring>
@@ -41,75 +40,6 @@ __global__ void __launch_bounds__(kBlock, 3) k_mc_props(McArgsT<S, double> A) {
     mc_props_cell<NS, CHEM>(A, n);
 }
 
-// The cells the surrogate leaves to the integrator (sur.ilist), G lanes per cell: the
-// lanes of a group evaluate the finite-difference Jacobian's columns side by side
-// (gas::ros2_advance_group), so the listed cells do not wait on serial integrations of one
-// lane each.  A short list (up to kChemShortList cells: latency-bound) takes 8 lanes per
-// cell, a long one 4 (the group's redundant factorisation then costs more than the
-// latency it saves); the choice is made on the device from the list's length.
-// The stiff integrator's iteration matrix in shared memory, m^2 doubles per thread of a block
-// (kernels over a compiled mechanism; m the unknowns of its iteration system, gas::SysMap: 9
-// for the H2/air mechanism, whose N2 is inert): two blocks of 128 threads per SM hold 162 kB,
-// where the thread's own array would live in local memory (its pivoted rows are indexed at
-// run time) and spill through L2; what the blocks leave of the SM's 256 kB serves as L1.
-constexpr bool kChemSharedMat = true;
-template <int NS, class KIN>
-constexpr size_t chem_smem_bytes() {
-    constexpr size_t m = gas::SysMap<KIN, NS + 1>::size;
-    return kChemSharedMat ? m * m * kBlock * sizeof(double) : 0;
-}
-constexpr unsigned kChemShortList = 5000;
-template <int NS, int G, typename S, class KIN, bool SMAT = false>
-__device__ __forceinline__ void chem_list_groups(const McArgsT<S, double> &A, unsigned cnt) {
-    const unsigned groups = gridDim.x * blockDim.x / G;
-    for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) / G; i < cnt; i += groups) {
-        const long n = A.sur.ilist[i];
-        double rho, rho_a[NS], Y[NS], T_si, rho_si, P_si;
-        mc_chem_state<NS>(A, n, rho, rho_a, Y, T_si, rho_si, P_si);
-        mc_chem_ros2<NS, McArgsT<S, double>, true, G, KIN, SMAT>(A, n, rho, rho_a, Y, T_si, rho_si, P_si, false);
-    }
-}
-// With a compiled mechanism (KIN: analytic species Jacobian, two right-hand sides per
-// sub-step besides it) a cell is one lane's work, its iteration matrix in shared memory as in
-// k_mc_chem (launched with chem_smem_bytes).
-template <int NS, typename S, class KIN = void>
-__global__ void __launch_bounds__(kBlock, 2) k_mc_chem_list(McArgsT<S, double> A) {
-    const unsigned cnt = *A.sur.icount;
-    if constexpr (!std::is_void_v<KIN>)
-        chem_list_groups<NS, 1, S, KIN, kChemSharedMat>(A, cnt);
-    else if (cnt <= kChemShortList)
-        chem_list_groups<NS, 8, S, KIN>(A, cnt);
-    else
-        chem_list_groups<NS, 4, S, KIN>(A, cnt);
-}
-
-// Chemistry of every fluid cell for LBMGPU_CHEM_ROSENBROCK handles, one thread per cell,
-// beside the transport part of the collision parameters (k_mc_props<CHEM_OFF>), from the
-// state the collision forms from the record (mc_chem_state):
-//   SUR = false: the stiff integrator (ROS2) itself;
-//   SUR = true : the surrogate's prediction where the gate passes it (element projection,
-//                output gate), the cells it does not cover and the audited ones appended
-//                to the integrator list for k_mc_chem_list.
-// A kernel of its own, so that its time (with the surrogate's kernels) is the chemistry's
-// share of the step, and the transport kernel keeps its own occupancy.
-// One thread per cell.  The integrator's vectors are sized by the species count at compile
-// time (ros2_advance_k) so that they stay in registers, two blocks per SM.  KIN: the compiled
-// kinetics of the handle's mechanism (gen_kinetics.py), void for the tables; with it the
-// iteration matrix of each thread lives in shared memory (kChemSharedMat), otherwise in the
-// thread's local memory.
-// The surrogate's instance (SUR: no integrator in it) holds far less per thread and runs four
-// blocks per SM.
-// PRED false: launched only while the surrogate's predictions are not in use (mode != 1).
-template <int NS, bool SUR, typename S, class KIN = void, bool PRED = true>
-__global__ void __launch_bounds__(kBlock, SUR ? 4 : 2) k_mc_chem(McArgsT<S, double> A) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
-    double rho, rho_a[NS], Y[NS], T_si, rho_si, P_si;
-    mc_chem_state<NS>(A, n, rho, rho_a, Y, T_si, rho_si, P_si);
-    constexpr bool smat = kChemSharedMat && !std::is_void_v<KIN>;
-    mc_chem_ros2<NS, McArgsT<S, double>, !SUR, 1, KIN, smat, PRED>(A, n, rho, rho_a, Y, T_si, rho_si, P_si, SUR);
-}
-
 // The energy-flux terms of the collision (mc_eflux_cell), after the collision parameters.
 template <int NS, typename S>
 __global__ void __launch_bounds__(kBlock) k_mc_eflux(McArgsT<S, double> A) {
@@ -130,15 +60,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_mc_relax(McArgsT<S, double> A) {
     else
         mc_relax_energy<NS>(A, n);
 }
-
-// the cells with a boundary upstream, one thread each (compact list)
-template <int NS, typename S>
-__global__ void __launch_bounds__(kBlock) k_mc_special(McArgsT<S, double> A, const long *__restrict__ blist) {
-    const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= A.nb) return;
-    mc_special_cell<NS>(A, blist[b], b);
-}
-
 
 // Interior cells (no boundary upstream): the pull of one population set per thread
 // (blockIdx.y = species, NS = the energy set) and its sums into the gsum planes --
@@ -296,37 +217,6 @@ __global__ void k_mc_pack(McArgsT<S, double> A, MixOff mo, SpOff so, char *__res
     for (int q = 0; q < 3; ++q) std_(mr, mo.energy_flux + 8 * q, q3[q]);
 }
 
-// The stiff chemistry over the compiled kinetics of the handle's mechanism, where the library
-// has them for it (kinetics_h2_air_9.cuh): every cell (k_mc_chem) or the integrator list
-// (k_mc_chem_list).  Returns false when the handle's mechanism is not compiled.
-template <int NS, typename S>
-bool launch_compiled_chem(lbmgpu *h, const McArgsT<S, double> &A, unsigned grid, bool list) {
-    if constexpr (NS == kin_h2_air_9::NS) {
-        using KinH2 = kin_h2_air_9::Kinetics;
-        if (h->kin != KIN_H2_AIR_9) return false;
-        constexpr size_t sm = chem_smem_bytes<NS, KinH2>();
-        // the launches below report a refused attribute as a launch error
-        if (list) {
-            if (sm > 48 * 1024)
-                (void)cudaFuncSetAttribute(k_mc_chem_list<NS, S, KinH2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sm);
-            k_mc_chem_list<NS, S, KinH2><<<grid, kBlock, sm, h->stream>>>(A);
-        } else if (A.sur.mode == 1) {
-            if (sm > 48 * 1024)
-                (void)cudaFuncSetAttribute(k_mc_chem<NS, false, S, KinH2>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_mc_chem<NS, false, S, KinH2><<<grid, kBlock, sm, h->stream>>>(A);
-        } else {
-            if (sm > 48 * 1024)
-                (void)cudaFuncSetAttribute(k_mc_chem<NS, false, S, KinH2, false>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_mc_chem<NS, false, S, KinH2, false><<<grid, kBlock, sm, h->stream>>>(A);
-        }
-        return true;
-    }
-    return false;
-}
-
 // The records of cells [c0, c1) -- the caller's arrays start at cell c0 -- into the device
 // state, one staging chunk at a time.
 template <int NS, typename S>
@@ -425,22 +315,12 @@ int collide_t(lbmgpu *h) {
     ev_end(h, ep);
     CK(cudaGetLastError());
     if (h->chem == CHEM_ROSENBROCK) {
-        EvPair ec{};
-        ev_begin(h, K_CHEM, ec);
-        if (A.sur.mode == 1 && A.sur.ilist)
-            k_mc_chem<NS, true, S><<<gp, kBlock, 0, h->stream>>>(A);
-        else if (!launch_compiled_chem<NS, S>(h, A, gp, false))
-            k_mc_chem<NS, false, S><<<gp, kBlock, 0, h->stream>>>(A);
-        ev_end(h, ec);
-        CK(cudaGetLastError());
-    }
-    if (A.sur.ilist) {
-        EvPair ei{};
-        ev_begin(h, K_SURROGATE, ei);
-        if (!launch_compiled_chem<NS, S>(h, A, 148 * 8, true))
-            k_mc_chem_list<NS, S><<<148 * 8, kBlock, 0, h->stream>>>(A);
-        ev_end(h, ei);
-        CK(cudaGetLastError());
+        McArgsT<double, double> C = base_args<double>(h);  // no populations in it: one instance for both storages
+        C.rec_cur = A.rec_cur;
+        C.rec_nxt = A.rec_nxt;
+        C.sur = A.sur;
+        const int rc_ = chem_step<NS>(h, C);
+        if (rc_) return rc_;
     }
     EvPair ee{};
     ev_begin(h, K_EFLUX, ee);
@@ -472,11 +352,8 @@ int stream_t(lbmgpu *h) {
         B.bst_nxt = bstb<S>(h, x);
         CK(cudaEventRecord(h->fork, h->stream));
         CK(cudaStreamWaitEvent(h->side, h->fork, 0));
-        EvPair eb{};
-        ev_begin(h, K_OTHER, eb, h->side);
-        k_mc_special<NS, S><<<(unsigned)((h->nb + 31) / 32), 32, 0, h->side>>>(B, h->blist);
-        ev_end(h, eb, h->side);
-        CK(cudaGetLastError());
+        const int rb = special_step<NS, S>(h, B);
+        if (rb) return rb;
         CK(cudaEventRecord(h->join, h->side));
     }
     EvPair ep{};

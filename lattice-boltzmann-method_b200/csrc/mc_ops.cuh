@@ -69,6 +69,19 @@ struct McOps {
     static constexpr int props_planes() { return lbm::pr_count<NS>(); }
     static constexpr int gsum_planes() { return lbm::gs_count<NS>(); }
 };
+// The stiff chemistry of one collision (mc_chem.cuh, instantiated in mc_chem<NS>.cu).
+template <int NS>
+int chem_step(lbmgpu *h, const lbm::McArgs &A);
+extern template int chem_step<9>(lbmgpu *, const lbm::McArgs &);
+extern template int chem_step<6>(lbmgpu *, const lbm::McArgs &);
+// The boundary cells of one streaming on the side stream (mc_special.cuh, instantiated in
+// mc_special<NS>.cu).
+template <int NS, typename S>
+int special_step(lbmgpu *h, const lbm::McArgsT<S, double> &A);
+extern template int special_step<9, double>(lbmgpu *, const lbm::McArgsT<double, double> &);
+extern template int special_step<9, float>(lbmgpu *, const lbm::McArgsT<float, double> &);
+extern template int special_step<6, double>(lbmgpu *, const lbm::McArgsT<double, double> &);
+extern template int special_step<6, float>(lbmgpu *, const lbm::McArgsT<float, double> &);
 extern template struct McOps<9>;
 extern template struct McOps<6>;
 
