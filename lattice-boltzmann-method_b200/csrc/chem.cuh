@@ -41,12 +41,9 @@ GAS_HD void reactor_rhs_k(const Tables &t, const RateT &K, double rho, const dou
 }
 
 // The reactor's right-hand side with NS species known at compile time, for the device's
-// one-thread-per-cell integrator: the temperature factors of each reaction evaluated inside
-// the reaction loop (no per-reaction arrays), log T taken once for the species entropies,
-// and the mass-action products and species sums over the dense stoichiometry tables, so that
-// every array is indexed by compile-time constants and stays in registers.  The same rate
-// laws as net_production; the products and sums run in species order instead of the order
-// the reaction lists its species, which moves results by rounding only.
+// one-thread-per-cell integrator: the rates by net_production_dense, log T taken once for the
+// species entropies, so that every array is indexed by compile-time constants and stays in
+// registers.
 template <int NS>
 GAS_HD void reactor_rhs_dense(const Tables &t, double rho, const double *y, double *F) {
     const lbmgpu_mech &m = t.m;
@@ -62,50 +59,8 @@ GAS_HD void reactor_rhs_dense(const Tables &t, double rho, const double *y, doub
         hRT[k] = a[0] + T * (a[1] / 2 + T * (a[2] / 3 + T * (a[3] / 4 + T * a[4] / 5))) + a[5] * invT;
         gRT[k] = hRT[k] - (a[0] * logT + T * (a[1] + T * (a[2] / 2 + T * (a[3] / 3 + T * a[4] / 4))) + a[6]);
         C[k] = rho * y[k] * t.invW[k];
-        w[k] = 0.0;
     }
-    for (int r = 0; r < m.n_reactions; ++r) {
-        double kf = m.A[r] * exp(m.b[r] * logT - m.Ea[r] * invRT);
-        double M = 1.0;
-        if (m.rtype[r] != LBMGPU_RXN_ELEMENTARY) {
-            M = 0.0;
-#pragma unroll
-            for (int k = 0; k < NS; ++k) M += m.eff[r][k] * C[k];
-        }
-        if (m.rtype[r] == LBMGPU_RXN_FALLOFF) {
-            const double k0 = m.A0[r] * exp(m.b0[r] * logT - m.Ea0[r] * invRT);
-            const double Pr = k0 * M / kf;
-            double F = 1.0;
-            if (m.troe_n[r] >= 3) {
-                const double a = m.troe[r][0], T3 = m.troe[r][1], T1 = m.troe[r][2];
-                double Fc = (1.0 - a) * exp(-T / T3) + a * exp(-T / T1);
-                if (m.troe_n[r] == 4) Fc += exp(-m.troe[r][3] * invT);
-                const double lFc = log10(fmax(Fc, 1e-300));
-                const double c = -0.4 - 0.67 * lFc, n = 0.75 - 1.27 * lFc;
-                const double lPr = log10(fmax(Pr, 1e-300));
-                const double x = (lPr + c) / (n - 0.14 * (lPr + c));
-                F = pow(10.0, lFc / (1.0 + x * x));
-            }
-            kf = kf * (Pr / (1.0 + Pr)) * F;
-            M = 1.0;
-        }
-        double fwd = kf * M, rev = 0.0;
-#pragma unroll
-        for (int k = 0; k < NS; ++k)
-            if (t.ord_f[r][k] != 0.0) fwd *= conc_pow(C[k], t.ord_f[r][k]);
-        if (m.reversible[r]) {
-            double dG = 0.0;
-#pragma unroll
-            for (int k = 0; k < NS; ++k) dG += t.nu_net[r][k] * gRT[k];
-            rev = kf * M * exp(dG - t.dnu[r] * log_cref);
-#pragma unroll
-            for (int k = 0; k < NS; ++k)
-                if (t.nu_b[r][k] != 0.0) rev *= conc_pow(C[k], t.nu_b[r][k]);
-        }
-        const double q = fwd - rev;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) w[k] += t.nu_net[r][k] * q;
-    }
+    net_production_dense<NS>(t, T, logT, invT, invRT, log_cref, gRT, C, w);
     double s = 0.0;
 #pragma unroll
     for (int k = 0; k < NS; ++k) {

@@ -82,6 +82,8 @@ struct Tables {
     double Ra_lat[MAXS];               // units.cp(R / W_a)
     double sqrt4W[MAXS][MAXS];         // sqrt(sqrt(W_b / W_a))   (Wilke factor, reference order)
     double wilke_den[MAXS][MAXS];      // sqrt(8 (1 + W_a / W_b))
+    double inv_wilke_den[MAXS][MAXS];  // its reciprocal, and W_a / W_b
+    double W_ratio[MAXS][MAXS];
     float inv_wilke_den_f[MAXS][MAXS]; // 1 / wilke_den and W_a / W_b in FP32 (the FP32 storage
     float W_ratio_f[MAXS][MAXS];       // mode's transport)
     // dense stoichiometry (species k of reaction r; 0 where k does not take part): reactant and
@@ -239,6 +241,29 @@ GAS_HD int T_from_u(const Tables &t, const double *Y, double u, double T0, doubl
     for (int it = 0; it < maxit; ++it) {
         const double f = int_energy_mass(t, Y, T) - u;
         const double cv = cv_mass(t, Y, T);
+        double dT = -f / cv;
+        if (dT > 500.0) dT = 500.0;
+        if (dT < -0.5 * T) dT = -0.5 * T;
+        T += dT;
+        if (fabs(dT) <= rtol * T) return it + 1;
+    }
+    return -1;
+}
+
+// T_from_u for NS species known at compile time: the same sums in the same order, unrolled, so
+// that Y stays in registers.
+template <int NS>
+GAS_HD int T_from_u_n(const Tables &t, const double *Y, double u, double T0, double rtol, int maxit, double &T) {
+    T = T0 > 0 ? T0 : 300.0;
+    for (int it = 0; it < maxit; ++it) {
+        double e = 0.0, c = 0.0;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            e += Y[k] * (h_RT_q(t, k, T) - 1.0) * t.invW[k];
+            c += Y[k] * (cp_R(t, k, T) - 1.0) * t.invW[k];
+        }
+        const double f = e * kR * T - u;
+        const double cv = c * kR;
         double dT = -f / cv;
         if (dT > 500.0) dT = 500.0;
         if (dT < -0.5 * T) dT = -0.5 * T;
@@ -465,6 +490,81 @@ GAS_HD void net_production(const Tables &t, double T, const double *C, double *w
     net_production_k(t, K, C, wdot);
 }
 
+// net_production for NS species known at compile time: each reaction's factors formed where it is
+// evaluated, its products and sums over the dense stoichiometry tables, so that every array is
+// indexed by compile-time constants; the products run in species order instead of the order
+// the reaction lists its species, which moves results by rounding only.  gRT: g_k/RT at T.
+template <int NS>
+GAS_HD void net_production_dense(const Tables &t, double T, double logT, double invT, double invRT, double log_cref,
+                                 const double *gRT, const double *C, double *w) {
+    const lbmgpu_mech &m = t.m;
+#pragma unroll
+    for (int k = 0; k < NS; ++k) w[k] = 0.0;
+    for (int r = 0; r < m.n_reactions; ++r) {
+        double kf = m.A[r] * exp(m.b[r] * logT - m.Ea[r] * invRT);
+        double M = 1.0;
+        if (m.rtype[r] != LBMGPU_RXN_ELEMENTARY) {
+            M = 0.0;
+#pragma unroll
+            for (int k = 0; k < NS; ++k) M += m.eff[r][k] * C[k];
+        }
+        if (m.rtype[r] == LBMGPU_RXN_FALLOFF) {
+            const double k0 = m.A0[r] * exp(m.b0[r] * logT - m.Ea0[r] * invRT);
+            const double Pr = k0 * M / kf;
+            double F = 1.0;
+            if (m.troe_n[r] >= 3) {
+                const double a = m.troe[r][0], T3 = m.troe[r][1], T1 = m.troe[r][2];
+                double Fc = (1.0 - a) * exp(-T / T3) + a * exp(-T / T1);
+                if (m.troe_n[r] == 4) Fc += exp(-m.troe[r][3] * invT);
+                const double lFc = log10(fmax(Fc, 1e-300));
+                const double c = -0.4 - 0.67 * lFc, n = 0.75 - 1.27 * lFc;
+                const double lPr = log10(fmax(Pr, 1e-300));
+                const double x = (lPr + c) / (n - 0.14 * (lPr + c));
+                F = pow(10.0, lFc / (1.0 + x * x));
+            }
+            kf = kf * (Pr / (1.0 + Pr)) * F;
+            M = 1.0;
+        }
+        double fwd = kf * M, rev = 0.0;
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+            if (t.ord_f[r][k] != 0.0) fwd *= conc_pow(C[k], t.ord_f[r][k]);
+        if (m.reversible[r]) {
+            double dG = 0.0;
+#pragma unroll
+            for (int k = 0; k < NS; ++k) dG += t.nu_net[r][k] * gRT[k];
+            rev = kf * M * exp(dG - t.dnu[r] * log_cref);
+#pragma unroll
+            for (int k = 0; k < NS; ++k)
+                if (t.nu_b[r][k] != 0.0) rev *= conc_pow(C[k], t.nu_b[r][k]);
+        }
+        const double q = fwd - rev;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) w[k] += t.nu_net[r][k] * q;
+    }
+}
+
+// The net production rates of NS species by net_production_dense, and of any mechanism by the
+// tables: the kinetics policies of the explicit chemistry scheme.
+template <int NS>
+struct DenseNet {
+    const Tables &t;
+    GAS_HD void operator()(double T, const double *C, double *w) const {
+        double gRT[NS];
+        const double logT = log(T);
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            const double *a = nasa(t, k, T);
+            gRT[k] = h_RT_q(t, k, T) - (a[0] * logT + T * (a[1] + T * (a[2] / 2 + T * (a[3] / 3 + T * a[4] / 4))) + a[6]);
+        }
+        net_production_dense<NS>(t, T, logT, 1.0 / T, 1.0 / (kR * T), log(kOneAtm / (kR * T)), gRT, C, w);
+    }
+};
+struct TableNet {
+    const Tables &t;
+    GAS_HD void operator()(double T, const double *C, double *w) const { net_production(t, T, C, w); }
+};
+
 // Least-squares polynomial fit (degree 4) of y(x) on n points; normal equations solved
 // by Gaussian elimination with partial pivoting (host, setup only).
 inline void polyfit4(const double *x, const double *y, int n, double *c) {
@@ -528,6 +628,8 @@ inline void make_tables(const lbmgpu_mech &m, Tables &t) {
             t.W_ratio_f[a][b] = (float)(m.W[a] / m.W[b]);
             t.wilke_den[a][b] = sqrt(8.0 * (1.0 + m.W[a] / m.W[b]));
             t.inv_wilke_den_f[a][b] = (float)(1.0 / t.wilke_den[a][b]);
+            t.inv_wilke_den[a][b] = 1.0 / t.wilke_den[a][b];
+            t.W_ratio[a][b] = m.W[a] / m.W[b];
         }
     for (int a = 0; a < t.ns; ++a) t.Ra_lat[a] = 0.0;
     for (int r = 0; r < MAXR; ++r) {

@@ -764,6 +764,394 @@ GAS_HD void rhs_t(const Thermo &th, double rho, const double *y, double *F) {
     F[9] = -es / (rho * cv);
 }
 
+// Net molar production rates w [kmol/m^3/s] at temperature T and concentrations C [kmol/m^3], from
+// the thermo th at T (gas::net_production, reaction by reaction).
+GAS_HD void net_t(const Thermo &th, double T, const double *C, double *w) {
+    const double logT = th.logT, invRT = th.invRT, log_cref = th.log_cref;
+    (void)T;
+    (void)logT;
+    (void)log_cref;
+    const double C0 = C[0];
+    const double C1 = C[1];
+    const double C2 = C[2];
+    const double C3 = C[3];
+    const double C4 = C[4];
+    const double C5 = C[5];
+    const double C6 = C[6];
+    const double C7 = C[7];
+    const double C8 = C[8];
+    double w0 = 0.0;
+    double w1 = 0.0;
+    double w2 = 0.0;
+    double w3 = 0.0;
+    double w4 = 0.0;
+    double w5 = 0.0;
+    double w6 = 0.0;
+    double w7 = 0.0;
+    double w8 = 0.0;
+    GAS_SCHED_FENCE();
+    {  // reaction 0
+        const double kf = 4.577000000000001e+16 * exp(-1.4 * logT - 436809600.0 * invRT);
+        const double er = exp((2.0 * th.gRT[1] - th.gRT[0]) - 1.0 * log_cref);
+        {  // rate of progress: 1 H2 <=> 2 H  + M
+            const double M = 2.5 * C0 + C1 + C2 + C3 + 12.0 * C4 + C5 + C6 + C7 + C8;
+            const double kfM = kf * M;
+            const double fwd = kfM * C0;
+            const double rev = kfM * er * (C1 * C1);
+            const double q = fwd - rev;
+            w0 -= q;
+            w1 += 2.0 * q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 1
+        const double kf = 50.80000000000001 * exp(2.67 * logT - 26325728.0 * invRT);
+        const double er = exp(th.gRT[1] + th.gRT[5] - th.gRT[0] - th.gRT[3]);
+        {  // rate of progress: 1 H2 + 1 O <=> 1 H + 1 OH
+            const double kfM = kf;
+            const double fwd = kfM * C0 * C3;
+            const double rev = kfM * er * C1 * C5;
+            const double q = fwd - rev;
+            w0 -= q;
+            w3 -= q;
+            w1 += q;
+            w5 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 2
+        const double kf = 43800000000.00001 * exp(-(29246160.0 * invRT));
+        const double er = exp(th.gRT[1] + th.gRT[4] - th.gRT[0] - th.gRT[5]);
+        {  // rate of progress: 1 H2 + 1 OH <=> 1 H + 1 H2O
+            const double kfM = kf;
+            const double fwd = kfM * C0 * C5;
+            const double rev = kfM * er * C1 * C4;
+            const double q = fwd - rev;
+            w0 -= q;
+            w5 -= q;
+            w1 += q;
+            w4 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 3
+        const double kf = 6165000000.000002 * exp(-0.5 * logT);
+        const double er = exp((th.gRT[2] - 2.0 * th.gRT[3]) - -1.0 * log_cref);
+        {  // rate of progress: 2 O <=> 1 O2  + M
+            const double M = 2.5 * C0 + C1 + C2 + C3 + 12.0 * C4 + C5 + C6 + C7 + C8;
+            const double kfM = kf * M;
+            const double fwd = kfM * (C3 * C3);
+            const double rev = kfM * er * C2;
+            const double q = fwd - rev;
+            w3 -= 2.0 * q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 4
+        const double kf = 114000000000.00003 * exp(-(63956624.0 * invRT));
+        const double er = exp(th.gRT[3] + th.gRT[5] - th.gRT[2] - th.gRT[1]);
+        {  // rate of progress: 1 O2 + 1 H <=> 1 O + 1 OH
+            const double kfM = kf;
+            const double fwd = kfM * C2 * C1;
+            const double rev = kfM * er * C3 * C5;
+            const double q = fwd - rev;
+            w2 -= q;
+            w1 -= q;
+            w3 += q;
+            w5 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 5
+        const double kf = 3.5000000000000016e+16 * exp(-2.0 * logT);
+        const double er = exp((th.gRT[4] - th.gRT[1] - th.gRT[5]) - -1.0 * log_cref);
+        {  // rate of progress: 1 H + 1 OH <=> 1 H2O  + M
+            const double M = 0.73 * C0 + C1 + C2 + C3 + 3.65 * C4 + C5 + C6 + C7 + C8;
+            const double kfM = kf * M;
+            const double fwd = kfM * C1 * C5;
+            const double rev = kfM * er * C4;
+            const double q = fwd - rev;
+            w1 -= q;
+            w5 -= q;
+            w4 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 6
+        const double kf = 67000.00000000001 * exp(1.704 * logT - 62704771.199999996 * invRT);
+        const double er = exp(2.0 * th.gRT[5] - th.gRT[3] - th.gRT[4]);
+        {  // rate of progress: 1 O + 1 H2O <=> 2 OH
+            const double kfM = kf;
+            const double fwd = kfM * C3 * C4;
+            const double rev = kfM * er * (C5 * C5);
+            const double q = fwd - rev;
+            w3 -= q;
+            w4 -= q;
+            w5 += 2.0 * q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 7
+        const double kf = 4714000000000.002 * exp(-1.0 * logT);
+        const double er = exp((th.gRT[5] - th.gRT[3] - th.gRT[1]) - -1.0 * log_cref);
+        {  // rate of progress: 1 O + 1 H <=> 1 OH  + M
+            const double M = 2.5 * C0 + C1 + C2 + C3 + 12.0 * C4 + C5 + C6 + C7 + C8;
+            const double kfM = kf * M;
+            const double fwd = kfM * C3 * C1;
+            const double rev = kfM * er * C5;
+            const double q = fwd - rev;
+            w3 -= q;
+            w1 -= q;
+            w5 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 8
+        const double kf = 2000000000000.0 * exp(0.9 * logT - 203965816.0 * invRT);
+        const double k0 = 2.4900000000000005e+21 * exp(-2.3 * logT - 203965816.0 * invRT);
+        const double lFc0 = -0.36653154442041347;
+        const double er = exp((2.0 * th.gRT[5] - th.gRT[6]) - 1.0 * log_cref);
+        {  // rate of progress: 1 H2O2 <=> 2 OH  (+M)
+            const double M = 3.7 * C0 + C1 + 1.2 * C2 + C3 + 7.65 * C4 + C5 + 7.7 * C6 + C7 + 1.5 * C8;
+            const double Pr = k0 * M / kf;
+            const double lFc = lFc0;
+            const double c = -0.4 - 0.67 * lFc, n = 0.75 - 1.27 * lFc;
+            const double lPr = log10(fmax(Pr, 1e-300));
+            const double x = (lPr + c) / (n - 0.14 * (lPr + c));
+            const double kfM = kf * (Pr / (1.0 + Pr)) * pow(10.0, lFc / (1.0 + x * x));
+            const double fwd = kfM * C6;
+            const double rev = kfM * er * (C5 * C5);
+            const double q = fwd - rev;
+            w6 -= q;
+            w5 += 2.0 * q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 9
+        const double kf = 24100000000.000008 * exp(-(16610480.0 * invRT));
+        const double er = exp(th.gRT[4] + th.gRT[5] - th.gRT[6] - th.gRT[1]);
+        {  // rate of progress: 1 H2O2 + 1 H <=> 1 H2O + 1 OH
+            const double kfM = kf;
+            const double fwd = kfM * C6 * C1;
+            const double rev = kfM * er * C4 * C5;
+            const double q = fwd - rev;
+            w6 -= q;
+            w1 -= q;
+            w4 += q;
+            w5 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 10
+        const double kf = 21500000.000000004 * exp(1.0 * logT - 25104000.0 * invRT);
+        const double er = exp(th.gRT[0] + th.gRT[7] - th.gRT[6] - th.gRT[1]);
+        {  // rate of progress: 1 H2O2 + 1 H <=> 1 H2 + 1 HO2
+            const double kfM = kf;
+            const double fwd = kfM * C6 * C1;
+            const double rev = kfM * er * C0 * C7;
+            const double q = fwd - rev;
+            w6 -= q;
+            w1 -= q;
+            w0 += q;
+            w7 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 11
+        const double kf = 9550.000000000002 * exp(2.0 * logT - 16610480.0 * invRT);
+        const double er = exp(th.gRT[5] + th.gRT[7] - th.gRT[6] - th.gRT[3]);
+        {  // rate of progress: 1 H2O2 + 1 O <=> 1 OH + 1 HO2
+            const double kfM = kf;
+            const double fwd = kfM * C6 * C3;
+            const double rev = kfM * er * C5 * C7;
+            const double q = fwd - rev;
+            w6 -= q;
+            w3 -= q;
+            w5 += q;
+            w7 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 12
+        const double kf = 1740000000.0000005 * exp(-(1330512.0 * invRT));
+        const double er = exp(th.gRT[4] + th.gRT[7] - th.gRT[6] - th.gRT[5]);
+        {  // rate of progress: 1 H2O2 + 1 OH <=> 1 H2O + 1 HO2
+            const double kfM = kf;
+            const double fwd = kfM * C6 * C5;
+            const double rev = kfM * er * C4 * C7;
+            const double q = fwd - rev;
+            w6 -= q;
+            w5 -= q;
+            w4 += q;
+            w7 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 13
+        const double kf = 75900000000.00002 * exp(-(30413496.0 * invRT));
+        const double er = exp(th.gRT[4] + th.gRT[7] - th.gRT[6] - th.gRT[5]);
+        {  // rate of progress: 1 H2O2 + 1 OH <=> 1 H2O + 1 HO2
+            const double kfM = kf;
+            const double fwd = kfM * C6 * C5;
+            const double rev = kfM * er * C4 * C7;
+            const double q = fwd - rev;
+            w6 -= q;
+            w5 -= q;
+            w4 += q;
+            w7 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 14
+        const double kf = 70790000000.00002 * exp(-(1234280.0 * invRT));
+        const double er = exp(2.0 * th.gRT[5] - th.gRT[7] - th.gRT[1]);
+        {  // rate of progress: 1 HO2 + 1 H <=> 2 OH
+            const double kfM = kf;
+            const double fwd = kfM * C7 * C1;
+            const double rev = kfM * er * (C5 * C5);
+            const double q = fwd - rev;
+            w7 -= q;
+            w1 -= q;
+            w5 += 2.0 * q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 15
+        const double kf = 11402000.000000002 * exp(1.0827 * logT - 2317015.52 * invRT);
+        const double er = exp(th.gRT[0] + th.gRT[2] - th.gRT[7] - th.gRT[1]);
+        {  // rate of progress: 1 HO2 + 1 H <=> 1 H2 + 1 O2
+            const double kfM = kf;
+            const double fwd = kfM * C7 * C1;
+            const double rev = kfM * er * C0 * C2;
+            const double q = fwd - rev;
+            w7 -= q;
+            w1 -= q;
+            w0 += q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 16
+        const double kf = 32500000000.000008;
+        const double er = exp(th.gRT[5] + th.gRT[2] - th.gRT[7] - th.gRT[3]);
+        {  // rate of progress: 1 HO2 + 1 O <=> 1 OH + 1 O2
+            const double kfM = kf;
+            const double fwd = kfM * C7 * C3;
+            const double rev = kfM * er * C5 * C2;
+            const double q = fwd - rev;
+            w7 -= q;
+            w3 -= q;
+            w5 += q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 17
+        const double kf = 7000000000.000002 * exp(-(-4572944.640000001 * invRT));
+        const double er = exp(th.gRT[4] + th.gRT[2] - th.gRT[5] - th.gRT[7]);
+        {  // rate of progress: 1 OH + 1 HO2 <=> 1 H2O + 1 O2
+            const double kfM = kf;
+            const double fwd = kfM * C5 * C7;
+            const double rev = kfM * er * C4 * C2;
+            const double q = fwd - rev;
+            w5 -= q;
+            w7 -= q;
+            w4 += q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 18
+        const double kf = 450000000000.0001 * exp(-(45729446.4 * invRT));
+        const double er = exp(th.gRT[4] + th.gRT[2] - th.gRT[5] - th.gRT[7]);
+        {  // rate of progress: 1 OH + 1 HO2 <=> 1 H2O + 1 O2
+            const double kfM = kf;
+            const double fwd = kfM * C5 * C7;
+            const double rev = kfM * er * C4 * C2;
+            const double q = fwd - rev;
+            w5 -= q;
+            w7 -= q;
+            w4 += q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 19
+        const double kf = 100000000000.00003 * exp(-(46195054.472 * invRT));
+        const double er = exp(th.gRT[6] + th.gRT[2] - 2.0 * th.gRT[7]);
+        {  // rate of progress: 2 HO2 <=> 1 H2O2 + 1 O2
+            const double kfM = kf;
+            const double fwd = kfM * (C7 * C7);
+            const double rev = kfM * er * C6 * C2;
+            const double q = fwd - rev;
+            w7 -= 2.0 * q;
+            w6 += q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 20
+        const double kf = 190000000.00000006 * exp(-(-5894941.3632 * invRT));
+        const double er = exp(th.gRT[6] + th.gRT[2] - 2.0 * th.gRT[7]);
+        {  // rate of progress: 2 HO2 <=> 1 H2O2 + 1 O2
+            const double kfM = kf;
+            const double fwd = kfM * (C7 * C7);
+            const double rev = kfM * er * C6 * C2;
+            const double q = fwd - rev;
+            w7 -= 2.0 * q;
+            w6 += q;
+            w2 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 21
+        const double kf = 4650000000.000001 * exp(0.44 * logT);
+        const double k0 = 17370000000000.006 * exp(-1.23 * logT);
+        const double lFc0 = -0.17392519729917352;
+        const double er = exp((th.gRT[7] - th.gRT[1] - th.gRT[2]) - -1.0 * log_cref);
+        {  // rate of progress: 1 H + 1 O2 <=> 1 HO2  (+M)
+            const double M = 1.3 * C0 + C1 + C2 + C3 + 10.0 * C4 + C5 + C6 + C7 + C8;
+            const double Pr = k0 * M / kf;
+            const double lFc = lFc0;
+            const double c = -0.4 - 0.67 * lFc, n = 0.75 - 1.27 * lFc;
+            const double lPr = log10(fmax(Pr, 1e-300));
+            const double x = (lPr + c) / (n - 0.14 * (lPr + c));
+            const double kfM = kf * (Pr / (1.0 + Pr)) * pow(10.0, lFc / (1.0 + x * x));
+            const double fwd = kfM * C1 * C2;
+            const double rev = kfM * er * C7;
+            const double q = fwd - rev;
+            w1 -= q;
+            w2 -= q;
+            w7 += q;
+        }
+    }
+    GAS_SCHED_FENCE();
+    {  // reaction 22
+        const double kf = 10000000000.000004;
+        const double er = exp((th.gRT[7] - th.gRT[3] - th.gRT[5]) - -1.0 * log_cref);
+        {  // rate of progress: 1 O + 1 OH <=> 1 HO2  + M
+            const double M = C0 + C1 + C2 + C3 + C4 + C5 + C6 + C7 + C8;
+            const double kfM = kf * M;
+            const double fwd = kfM * C3 * C5;
+            const double rev = kfM * er * C7;
+            const double q = fwd - rev;
+            w3 -= q;
+            w5 -= q;
+            w7 += q;
+        }
+    }
+    w[0] = w0;
+    w[1] = w1;
+    w[2] = w2;
+    w[3] = w3;
+    w[4] = w4;
+    w[5] = w5;
+    w[6] = w6;
+    w[7] = w7;
+    w[8] = w8;
+}
+
 // rhs_t, and s times the Jacobian of F with respect to (Y, T) at fixed density over the
 // unknowns of the integrator's iteration system (Kinetics::sys_full): J(p, q) = s dF_a / dY_b,
 // a = sys_full(p), b = sys_full(q), the temperature the last unknown.
@@ -2243,6 +2631,12 @@ struct Kinetics {
     GAS_HD static constexpr int sys_full(int i) { return i == 0 ? 0 : (i == 1 ? 1 : (i == 2 ? 2 : (i == 3 ? 3 : (i == 4 ? 4 : (i == 5 ? 5 : (i == 6 ? 6 : (i == 7 ? 7 : (9)))))))); }
     GAS_HD void factors(double T, Thermo &k) const { thermo(T, k); }
     GAS_HD void rhs(const Thermo &k, double rho, const double *y, double *F) const { rhs_t(k, rho, y, F); }
+    // net production rates at (T, C): the explicit scheme's policy
+    GAS_HD void operator()(double T, const double *C, double *w) const {
+        Thermo th;
+        thermo(T, th);
+        net_t(th, T, C, w);
+    }
     template <class Mat>
     GAS_HD void rhs_jacobian(const Thermo &k, double rho, const double *y, double *F, double s, Mat &J) const {
         rhs_jac(k, rho, y, F, s, J);

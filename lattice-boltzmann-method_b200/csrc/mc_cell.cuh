@@ -43,6 +43,11 @@
 namespace lbm {
 
 constexpr double kSpeciesMin = 1e-8;   // SPECIES_MIN, src/headers/defines.hpp:96
+#if defined(__CUDA_ARCH__)
+constexpr bool kHostBuild = false;
+#else
+constexpr bool kHostBuild = true;
+#endif
 
 enum : int {
     RM_RHO = 0, RM_U = 1, RM_V = 2, RM_W = 3, RM_T = 4, RM_P = 5, RM_RHOE = 6, RM_P00 = 7,  // P00 P01 P02 P11 P12 P22
@@ -197,14 +202,18 @@ MC_HD long pull_idx(const McPull &p, int l) { return p.X[cidx(cx(l))] + p.Y[cidx
 template <int NS>
 MC_HD double set_mass_fractions(const gas::Tables &t, const double *y, double *Y, double *X) {
     double s = 0.0;
+#pragma unroll
     for (int k = 0; k < NS; ++k) {
         Y[k] = y[k] > 0.0 ? y[k] : 0.0;
         s += Y[k];
     }
+#pragma unroll
     for (int k = 0; k < NS; ++k) Y[k] /= s;
     double sw = 0.0;
+#pragma unroll
     for (int k = 0; k < NS; ++k) sw += Y[k] / t.m.W[k];
     const double W = 1.0 / sw;
+#pragma unroll
     for (int k = 0; k < NS; ++k) X[k] = Y[k] / t.m.W[k] * W;
     return W;
 }
@@ -214,17 +223,20 @@ MC_HD double set_mass_fractions(const gas::Tables &t, const double *y, double *Y
 template <int NS>
 MC_HD double set_mass_fractions_fast(const gas::Tables &t, const double *y, double *Y, double *X) {
     double s = 0.0;
+#pragma unroll
     for (int k = 0; k < NS; ++k) {
         Y[k] = y[k] > 0.0 ? y[k] : 0.0;
         s += Y[k];
     }
     const double is = 1.0 / s;
     double sw = 0.0;
+#pragma unroll
     for (int k = 0; k < NS; ++k) {
         Y[k] *= is;
         sw += Y[k] * t.invW[k];
     }
     const double W = 1.0 / sw;
+#pragma unroll
     for (int k = 0; k < NS; ++k) X[k] = Y[k] * t.invW[k] * W;
     return W;
 }
@@ -232,25 +244,30 @@ MC_HD double set_mass_fractions_fast(const gas::Tables &t, const double *y, doub
 // The face-difference terms a cell offers its neighbours: species Q_{a,d} with the species
 // gas constant (src/lbm-collision.cpp:487-489) and the mixture Q_d with the composition
 // gas constant a neighbour uses (src/lbm-collision.cpp:207-215, 296-300; zero gas constant
-// for cells that are not fluid-like).
-template <int NS, class AT>
+// for cells that are not fluid-like).  FAST: products by reciprocals (the FP32 storage mode).
+template <int NS, bool FAST = false, class AT>
 MC_HD void store_face_terms(const AT &A, typename AT::R *R, long n, int ty, double rho, const double u[3], double T,
                             const double *rho_a, const double (*ua)[3]) {
     const gas::Tables &t = *A.tab;
     double gc = 0.0;
     if (fluid_like(ty)) {
+        const double ir = FAST ? 1.0 / rho : 0.0;
         double sYW = 0.0, sY = 0.0;
+#pragma unroll
         for (int a = 0; a < NS; ++a) {
-            const double Ya = rho_a[a] / rho;
-            sYW += Ya / t.m.W[a];
+            const double Ya = FAST ? rho_a[a] * ir : rho_a[a] / rho;
+            sYW += FAST ? Ya * t.invW[a] : Ya / t.m.W[a];
             sY += Ya;
         }
         gc = (double)u_cp(A.U, (float)(gas::kR * sYW / sY));
     }
+#pragma unroll
     for (int d = 0; d < 3; ++d)
         put(A, R, RM_QX + d, n, rho * u[d] * (1.0 - 3.0 * gc * T) - rho * (u[d] * u[d] * u[d]));
+#pragma unroll
     for (int a = 0; a < NS; ++a) {
         const double Ra = t.Ra_lat[a];
+#pragma unroll
         for (int d = 0; d < 3; ++d)
             put(A, R, rs(a, RS_QX + d), n,
                 rho_a[a] * ua[a][d] * (1.0 - 3.0 * Ra * T) - rho_a[a] * (ua[a][d] * ua[a][d] * ua[a][d]));
@@ -353,10 +370,14 @@ template <int NS, typename C>
 MC_HD void mc_stefan_maxwell(int dt, double p_old, const double *Xold, const double *rho_s, const double (*j_a)[3],
                              double (*Ld)[NS], double (*usm)[3]) {
     C L[NS][NS];
+#pragma unroll
     for (int a = 0; a < NS; ++a)
+#pragma unroll
         for (int b = 0; b < a; ++b) L[a][b] = (C)Ld[a][b];
+#pragma unroll
     for (int a = 0; a < NS; ++a) {
         C d = (C)(rho_s[a] == 0.0 ? 1.0 : rho_s[a]);
+#pragma unroll
         for (int b = 0; b < NS; ++b) {
             if (b == a) continue;
             const C D = b < a ? L[a][b] : L[b][a];
@@ -366,28 +387,38 @@ MC_HD void mc_stefan_maxwell(int dt, double p_old, const double *Xold, const dou
         }
         L[a][a] = d;
     }
+#pragma unroll
     for (int c = 0; c < NS; ++c) {  // in-place lower Cholesky factor
         C d = L[c][c];
+#pragma unroll
         for (int q = 0; q < c; ++q) d -= L[c][q] * L[c][q];
         L[c][c] = sqrt(d);
+#pragma unroll
         for (int r = c + 1; r < NS; ++r) {
             C s = L[r][c];
+#pragma unroll
             for (int q = 0; q < c; ++q) s -= L[r][q] * L[c][q];
             L[r][c] = s / L[c][c];
         }
     }
+#pragma unroll
     for (int dmn = 0; dmn < 3; ++dmn) {
         C y[NS], x[NS];
+#pragma unroll
         for (int r = 0; r < NS; ++r) {
             C s = (C)j_a[r][dmn];
+#pragma unroll
             for (int q = 0; q < r; ++q) s -= L[r][q] * y[q];
             y[r] = s / L[r][r];
         }
+#pragma unroll
         for (int r = NS - 1; r >= 0; --r) {
             C s = y[r];
+#pragma unroll
             for (int q = r + 1; q < NS; ++q) s -= L[q][r] * x[q];
             x[r] = s / L[r][r];
         }
+#pragma unroll
         for (int r = 0; r < NS; ++r) usm[r][dmn] = (double)x[r];
     }
 }
@@ -482,12 +513,16 @@ MC_HDN void mc_moments_finish(const AT &A, long n, const Sums &S) {
     // the diffusion coefficients first (one load per pair, into the lower triangle that
     // the Stefan-Maxwell entries then replace row by row), the momenta next
     double L[NS][NS];  // lower triangle and diagonal only
+#pragma unroll
     for (int a = 0; a < NS; ++a)
+#pragma unroll
         for (int b = 0; b < a; ++b) L[a][b] = A.props[(long)pr_d<NS>(a, b) * A.ncell + n];
     double j_a[NS][3];
     double rho = 0, ru = 0, rv = 0, rw = 0, rho_s[NS];
+#pragma unroll
     for (int a = 0; a < NS; ++a) {
         const double ra = S.rho_a(a);
+#pragma unroll
         for (int d = 0; d < 3; ++d) j_a[a][d] = S.j(a, d);
         rho_s[a] = ra > kSpeciesMin ? ra : kSpeciesMin;
         rho += ra;
@@ -501,6 +536,7 @@ MC_HDN void mc_moments_finish(const AT &A, long n, const Sums &S) {
     // this step evaluated at the same old state (T, p, Y)
     const double p_old = rec(A, A.rec_cur, RM_P, n);
     double Xold[NS];
+#pragma unroll
     for (int a = 0; a < NS; ++a) Xold[a] = rec(A, A.rec_cur, rs(a, RS_X), n);
     // FP64 in both storage modes (an FP32 solve moved the characteristic-inflow case's
     // temperature by 2e-5 against FP64 within 20 steps -- its boundary cells amplify last-bit
@@ -519,22 +555,25 @@ MC_HDN void mc_moments_finish(const AT &A, long n, const Sums &S) {
     double Wn;
     if constexpr (fast) {
         const double ir = 1.0 / rho;
+#pragma unroll
         for (int a = 0; a < NS; ++a) Yr[a] = rho_s[a] * ir;
         Wn = set_mass_fractions_fast<NS>(t, Yr, Y, X);
     } else {
+#pragma unroll
         for (int a = 0; a < NS; ++a) Yr[a] = rho_s[a] / rho;
         Wn = set_mass_fractions<NS>(t, Yr, Y, X);
     }
     const double rhoe = S.rhoe();
     double e = rhoe / rho;
+#pragma unroll
     for (int a = 0; a < NS; ++a)
-        e = e - 0.5 * rho_s[a] / rho * (usm[a][0] * usm[a][0] + usm[a][1] * usm[a][1] + usm[a][2] * usm[a][2]);
+        e = e - 0.5 * Yr[a] * (usm[a][0] * usm[a][0] + usm[a][1] * usm[a][1] + usm[a][2] * usm[a][2]);
     const double u_si = si_energy_mass(A.U, (float)e);
     const double vol = 1.0 / (double)si_rho(A.U, (float)rho);
     const double rho_n_si = 1.0 / vol;
     double Tn;
     const int it = fast ? gas::T_from_u_fast<NS>(t, Y, u_si, T_si, 1e-14, 100, Tn)
-                        : gas::T_from_u(t, Y, u_si, T_si, 1e-14, 100, Tn);
+                        : gas::T_from_u_n<NS>(t, Y, u_si, T_si, 1e-14, 100, Tn);
     if (it < 0) atomic_status(A.status, LBMGPU_ST_NEWTON);
     const double Pn = rho_n_si * gas::kR * Tn / Wn;
     const double Tl = u_temp(A.U, (float)Tn);
@@ -547,14 +586,17 @@ MC_HDN void mc_moments_finish(const AT &A, long n, const Sums &S) {
     put(A, R, RM_T, n, Tl);
     put(A, R, RM_P, n, u_p(A.U, (float)Pn));
     put(A, R, RM_RHOE, n, rhoe);
+#pragma unroll
     for (int q = 0; q < 6; ++q) put(A, R, RM_P00 + q, n, S.P6(q));
+#pragma unroll
     for (int a = 0; a < NS; ++a) {
         put(A, R, rs(a, RS_RHO), n, rho_s[a]);
+#pragma unroll
         for (int d = 0; d < 3; ++d) put(A, R, rs(a, RS_UX + d), n, usm[a][d]);
         put(A, R, rs(a, RS_X), n, X[a]);
     }
     const double um[3] = {u, v, w};
-    store_face_terms<NS>(A, R, n, T_F, rho, um, Tl, rho_s, usm);
+    store_face_terms<NS, fast>(A, R, n, T_F, rho, um, Tl, rho_s, usm);
     if (!isfinite(rho) || !isfinite(Tn) || !isfinite(u) || !isfinite(v) || !isfinite(w))
         atomic_status(A.status, LBMGPU_ST_NAN);
     else if (!(rho > 0.0) || !(Tn > 0.0))
@@ -748,72 +790,86 @@ MC_HD void mc_chem_state(const AT &A, long n, double &rho, double *rho_a, double
 }
 
 // The transport part of the collision parameters (lbm-collision.cpp:402-471 species rates and
-// Maxwell-Stefan force, :231-316 energy rates) in FP64, the reference's arithmetic and order
-// (the FP64 storage mode, bit-faithful).
+// Maxwell-Stefan force, :231-316 energy rates) in FP64 (the FP64 storage mode).  The quotients that
+// the reference rounds to float at its unit conversions stay divisions, so their floats are the
+// reference's.  The Wilke pairs multiply per-species square roots and reciprocals on the device
+// (45 pairs: 18 square roots and reciprocals in place of 225; rounding-level differences, as its exp
+// and log make them anyway); the host build, which restates the reference operation by operation,
+// keeps the quotients.  Every loop is unrolled: the arrays live in registers.
 template <int NS, class AT>
-MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a, const double (*ua)[3],
-                             const double *Xs, const double *Y, const double *X, double W, double T_si, double P_si,
-                             double Uint) {
+MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a, const double *Y, const double *X,
+                             double W, double T_si, double P_si, double Uint) {
     const gas::Tables &t = *A.tab;
+    const typename AT::R *Rc = A.rec_cur;
     double *Pr = A.props;
     auto prp = [&](int plane, double v) { Pr[(long)plane * A.ncell + n] = v; };
     const double dt = A.dt;
+    const double xT = gas::lnT_x(T_si);
+    double Xs[NS];  // the record's mole fractions
+#pragma unroll
+    for (int a = 0; a < NS; ++a) Xs[a] = rec(A, Rc, rs(a, RS_X), n);
     // -- species viscosities; Wilke weights phi_ab = (1 + sqrt(mu_a/mu_b) (W_b/W_a)^1/4)^2 /
     // sqrt(8 (1 + W_a/W_b)) formed for b >= a and mirrored, phi_ba = mu_b/mu_a W_a/W_b phi_ab
     // (lbm-collision.cpp:402-430).  Each weight enters the two row sums the reference forms
     // with it -- sum_b Xs_b phi_ab for the species rates, sum_b X_b phi_ab for the mixture
     // viscosity -- pair by pair; every row still receives its terms in the order b = 0..NS-1.
-    const double xT = gas::lnT_x(T_si);
-    double mu_k[NS];
-    for (int a = 0; a < NS; ++a) mu_k[a] = gas::species_visc_x(t, a, xT);
-    double den_s[NS], den_m[NS];
-    for (int a = 0; a < NS; ++a) den_s[a] = den_m[a] = 0.0;
-    for (int a = 0; a < NS; ++a)
-        for (int b = a; b < NS; ++b) {
-            const double f1 = 1.0 + sqrt(mu_k[a] / mu_k[b]) * t.sqrt4W[a][b];
-            const double pab = f1 * f1 / t.wilke_den[a][b];
-            const double pba = mu_k[b] / mu_k[a] * t.m.W[a] / t.m.W[b] * pab;
-            if (b == a) {
-                den_s[a] = den_s[a] + Xs[a] * pba;
-                den_m[a] += X[a] * pba;
-            } else {
-                den_s[a] = den_s[a] + Xs[b] * pab;
-                den_m[a] += X[b] * pab;
-                den_s[b] = den_s[b] + Xs[a] * pba;
-                den_m[b] += X[a] * pba;
-            }
+    double mu = 0.0;  // Wilke mixture viscosity sum_k X_k mu_k / sum_j X_j phi_kj
+    {
+        double mu_k[NS], smu[NS], ismu[NS];
+#pragma unroll
+        for (int a = 0; a < NS; ++a) {
+            mu_k[a] = gas::species_visc_x(t, a, xT);
+            smu[a] = sqrt(mu_k[a]);
+            ismu[a] = 1.0 / smu[a];
         }
-    for (int a = 0; a < NS; ++a) {
-        const double visc = Xs[a] * (double)u_mu(A.U, (float)mu_k[a]) / den_s[a];
-        prp(pr_om<NS>(a), 2 * Xs[a] * p * dt / (Xs[a] * p * dt + 2 * visc));
+        double den_s[NS], den_m[NS];
+#pragma unroll
+        for (int a = 0; a < NS; ++a) den_s[a] = den_m[a] = 0.0;
+#pragma unroll
+        for (int a = 0; a < NS; ++a)
+#pragma unroll
+            for (int b = a; b < NS; ++b) {
+                double pab, pba;
+                if (kHostBuild) {
+                    const double f1 = 1.0 + sqrt(mu_k[a] / mu_k[b]) * t.sqrt4W[a][b];
+                    pab = f1 * f1 / t.wilke_den[a][b];
+                    pba = mu_k[b] / mu_k[a] * t.m.W[a] / t.m.W[b] * pab;
+                } else {
+                    const double f1 = 1.0 + smu[a] * ismu[b] * t.sqrt4W[a][b], r = smu[b] * ismu[a];
+                    pab = f1 * f1 * t.inv_wilke_den[a][b];
+                    pba = r * r * t.W_ratio[a][b] * pab;
+                }
+                if (b == a) {
+                    den_s[a] += Xs[a] * pba;
+                    den_m[a] += X[a] * pba;
+                } else {
+                    den_s[a] += Xs[b] * pab;
+                    den_m[a] += X[b] * pab;
+                    den_s[b] += Xs[a] * pba;
+                    den_m[b] += X[a] * pba;
+                }
+            }
+#pragma unroll
+        for (int a = 0; a < NS; ++a) {
+            const double visc = Xs[a] * (double)u_mu(A.U, (float)mu_k[a]) / den_s[a];
+            prp(pr_om<NS>(a), 2 * Xs[a] * p * dt / (Xs[a] * p * dt + 2 * visc));
+            mu += X[a] * mu_k[a] / den_m[a];
+        }
     }
-
-    // -- Maxwell-Stefan force (lbm-collision.cpp:433-471); the diagonal term vanishes
-    double F[NS][3];
-    for (int a = 0; a < NS; ++a)
-        for (int d = 0; d < 3; ++d) F[a][d] = 0.0;
-    for (int a = 0; a < NS; ++a)
-        for (int b = 0; b < a; ++b) {
-            const double D = u_nu(A.U, (float)gas::binary_diff_x(t, a, b, xT, P_si));
-            prp(pr_d<NS>(a, b), D);
-            // the reference's -p X_a X_b / D_ab, once per ordered pair
-            const double kab = -1.0 * p * Xs[a] * Xs[b] / D, kba = -1.0 * p * Xs[b] * Xs[a] / D;
-            for (int d = 0; d < 3; ++d) {
-                F[a][d] += kab * (ua[a][d] - ua[b][d]);
-                F[b][d] += kba * (ua[b][d] - ua[a][d]);
-            }
-        }
-    for (int a = 0; a < NS; ++a)
-        for (int d = 0; d < 3; ++d) prp(pr_f<NS>(a, d), F[a][d] * dt / rho_a[a]);
-
     // -- energy collision parameters (lbm-collision.cpp:231-316): the relaxation rates here,
     // the energy-flux terms (neighbour differences) in mc_eflux_cell
-    double mu = 0.0;  // Wilke mixture viscosity sum_k X_k mu_k / sum_j X_j phi_kj
-    for (int k = 0; k < NS; ++k) mu += X[k] * mu_k[k] / den_m[k];
-    const double cp = u_cp(A.U, (float)gas::cp_mass(t, Y, T_si));
+    double cpm = 0.0, s1 = 0.0, s2 = 0.0;  // c_p; Mathur-Saxena conductivity
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+        cpm += Y[k] * gas::cp_R(t, k, T_si) * t.invW[k];
+        const double lk = gas::species_cond_x(t, k, xT);
+        s1 += X[k] * lk;
+        s2 += X[k] / lk;
+    }
+    const double cp = u_cp(A.U, (float)(cpm * gas::kR));
     const double gasconstant = u_cp(A.U, (float)(gas::kR / W));
     mu = u_mu(A.U, (float)mu);
-    const double lam = u_cond(A.U, (float)gas::mix_cond(t, X, T_si, P_si, mu_k));
+    const double lam = u_cond(A.U, (float)(0.5 * (s1 + 1.0 / s2)));
     const double theta = u_energy_mass(A.U, (float)(gas::kR * T_si / W));
     const double om1 = 2 * p * cp * dt / (p * cp * dt + 2 * lam);
     const double om = 2 * p * dt / (p * dt + 2 * mu);
@@ -823,6 +879,38 @@ MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a,
     prp(pr_theta<NS>(), theta);
     prp(pr_uint<NS>(), Uint);
     prp(pr_gc<NS>(), gasconstant);
+
+    // -- Maxwell-Stefan force (lbm-collision.cpp:433-471); the diagonal term vanishes
+    double ua[NS][3], F[NS][3];
+#pragma unroll
+    for (int a = 0; a < NS; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            ua[a][d] = rec(A, Rc, rs(a, RS_UX + d), n);
+            F[a][d] = 0.0;
+        }
+#pragma unroll
+    for (int a = 0; a < NS; ++a)
+#pragma unroll
+        for (int b = 0; b < a; ++b) {
+            const double D = u_nu(A.U, (float)gas::binary_diff_x(t, a, b, xT, P_si));
+            prp(pr_d<NS>(a, b), D);
+            // the reference's -p X_a X_b / D_ab, per ordered pair in the host build
+            const double kab = -1.0 * p * Xs[a] * Xs[b] / D;
+            const double kba = kHostBuild ? -1.0 * p * Xs[b] * Xs[a] / D : kab;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double du = ua[a][d] - ua[b][d];
+                F[a][d] += kab * du;
+                F[b][d] -= kba * du;
+            }
+        }
+#pragma unroll
+    for (int a = 0; a < NS; ++a) {
+        const double s = dt / rho_a[a];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) prp(pr_f<NS>(a, d), kHostBuild ? F[a][d] * dt / rho_a[a] : F[a][d] * s);
+    }
 }
 
 // The same parameters for the FP32 storage mode, in FP32 arithmetic: species viscosities,
@@ -832,9 +920,8 @@ MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a,
 // in FP64 (its terms are differences of nearly equal species velocities).  The Wilke pairs
 // take products of per-species square roots and reciprocals in place of the quotients.
 template <int NS, class AT>
-MC_HDN void mc_transport_f32(const AT &A, long n, double p, const double *rho_a, const double (*ua)[3],
-                             const double *Xs, const double *Y, const double *X, double W, double T_si, double P_si,
-                             double Uint) {
+MC_HDN void mc_transport_f32(const AT &A, long n, double p, const double *rho_a, const double *Y, const double *X,
+                             double W, double T_si, double P_si, double Uint) {
     const gas::Tables &t = *A.tab;
     double *Pr = A.props;
     auto prp = [&](int plane, double v) { Pr[(long)plane * A.ncell + n] = v; };
@@ -849,7 +936,7 @@ MC_HDN void mc_transport_f32(const AT &A, long n, double p, const double *rho_a,
         imu[a] = 1.f / mu_k[a];
         smu[a] = sqrtf(mu_k[a]);
         ismu[a] = 1.f / smu[a];
-        Xsf[a] = (float)Xs[a];
+        Xsf[a] = (float)rec(A, A.rec_cur, rs(a, RS_X), n);
         Xf[a] = (float)X[a];
     }
     float den_s[NS], den_m[NS];
@@ -877,32 +964,6 @@ MC_HDN void mc_transport_f32(const AT &A, long n, double p, const double *rho_a,
         const float visc = Xsf[a] * u_mu(A.U, mu_k[a]) / den_s[a];
         prp(pr_om<NS>(a), (double)(2.f * Xsf[a] * pf * dt / (Xsf[a] * pf * dt + 2.f * visc)));
     }
-    double F[NS][3];
-#pragma unroll
-    for (int a = 0; a < NS; ++a)
-#pragma unroll
-        for (int d = 0; d < 3; ++d) F[a][d] = 0.0;
-    const float inv_P = 1.f / (float)P_si;
-#pragma unroll
-    for (int a = 0; a < NS; ++a)
-#pragma unroll
-        for (int b = 0; b < a; ++b) {
-            const float D = u_nu(A.U, expf(gas::fit_eval_f(t.fit_diff[a][b], xT)) * inv_P);
-            prp(pr_d<NS>(a, b), (double)D);
-            const double k = (double)(-pf * Xsf[a] * Xsf[b] / D);
-#pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const double du = ua[a][d] - ua[b][d];
-                F[a][d] += k * du;
-                F[b][d] -= k * du;
-            }
-        }
-#pragma unroll
-    for (int a = 0; a < NS; ++a) {
-        const double s = (double)dt / rho_a[a];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) prp(pr_f<NS>(a, d), F[a][d] * s);
-    }
     float mu = 0.f, cpm = 0.f, s1 = 0.f, s2 = 0.f;
     const float Tf = (float)T_si;
 #pragma unroll
@@ -928,83 +989,141 @@ MC_HDN void mc_transport_f32(const AT &A, long n, double p, const double *rho_a,
     prp(pr_theta<NS>(), theta);
     prp(pr_uint<NS>(), Uint);
     prp(pr_gc<NS>(), (double)gasconstant);
+    double ua[NS][3], F[NS][3];
+#pragma unroll
+    for (int a = 0; a < NS; ++a)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            ua[a][d] = rec(A, A.rec_cur, rs(a, RS_UX + d), n);
+            F[a][d] = 0.0;
+        }
+    const float inv_P = 1.f / (float)P_si;
+#pragma unroll
+    for (int a = 0; a < NS; ++a)
+#pragma unroll
+        for (int b = 0; b < a; ++b) {
+            const float D = u_nu(A.U, expf(gas::fit_eval_f(t.fit_diff[a][b], xT)) * inv_P);
+            prp(pr_d<NS>(a, b), (double)D);
+            const double k = (double)(-pf * Xsf[a] * Xsf[b] / D);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double du = ua[a][d] - ua[b][d];
+                F[a][d] += k * du;
+                F[b][d] -= k * du;
+            }
+        }
+#pragma unroll
+    for (int a = 0; a < NS; ++a) {
+        const double s = (double)dt / rho_a[a];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) prp(pr_f<NS>(a, d), F[a][d] * s);
+    }
 }
 
+// internal energy per mass without the species kinetic energy (lbm-collision.cpp:260-263,
+// 373-376); Yr = rho_a / rho (half of it is the reference's quotient of the halved density)
+template <int NS, class AT>
+MC_HD double mc_u_int(const AT &A, long n, double rho, const double *Yr) {
+    const typename AT::R *Rc = A.rec_cur;
+    double U = rec(A, Rc, RM_RHOE, n) / rho;
+#pragma unroll
+    for (int a = 0; a < NS; ++a) {
+        const double u = rec(A, Rc, rs(a, RS_UX), n), v = rec(A, Rc, rs(a, RS_UX + 1), n),
+                     w = rec(A, Rc, rs(a, RS_UX + 2), n);
+        U = U - 0.5 * Yr[a] * (u * u + v * v + w * w);
+    }
+    return U;
+}
+
+// The state the collision forms from the record (Cantera's setMassFractions + setState_TD,
+// lbm-collision.cpp:364-367 and :236-238); the FP32 storage mode takes the reciprocal forms
+// (rounding-level differences, as in its moment solve).  Yr: rho_a / rho.  Returns the molar mass.
+template <int NS, class AT>
+MC_HD double mc_state(const AT &A, double rho, const double *rho_a, double *Yr, double *Y, double *X) {
+    const gas::Tables &t = *A.tab;
+    if constexpr (sizeof(typename AT::P) == sizeof(float)) {
+        const double ir = 1.0 / rho;
+#pragma unroll
+        for (int a = 0; a < NS; ++a) Yr[a] = rho_a[a] * ir;
+        return set_mass_fractions_fast<NS>(t, Yr, Y, X);
+    } else {
+#pragma unroll
+        for (int a = 0; a < NS; ++a) Yr[a] = rho_a[a] / rho;
+        return set_mass_fractions<NS>(t, Yr, Y, X);
+    }
+}
+
+// The reference's chemistry: two explicit half steps with T from (u, v) in between
+// (lbm-collision.cpp:370-399).  `net`: the net production rates at (T, C).
+template <int NS, class Net, class AT>
+MC_HDN void mc_chem_explicit(const AT &A, long n, const Net &net) {
+    const gas::Tables &t = *A.tab;
+    const typename AT::R *Rc = A.rec_cur;
+    const double rho = rec(A, Rc, RM_RHO, n), dt = A.dt;
+    double rho_a[NS], Yr[NS], Y[NS], X[NS];
+#pragma unroll
+    for (int a = 0; a < NS; ++a) rho_a[a] = rec(A, Rc, rs(a, RS_RHO), n);
+    (void)mc_state<NS>(A, rho, rho_a, Yr, Y, X);
+    const double u_si = si_energy_mass(A.U, (float)mc_u_int<NS>(A, n, rho, Yr));
+    const double vol = 1.0 / (double)si_rho(A.U, (float)rho);
+    double T = si_temp(A.U, (float)rec(A, Rc, RM_T, n)), rc = si_rho(A.U, (float)rho), drho[NS];
+#pragma unroll
+    for (int a = 0; a < NS; ++a) drho[a] = 0.0;
+#pragma unroll 1
+    for (int sub = 0; sub < 2; ++sub) {
+        double C[NS], wd[NS];
+#pragma unroll
+        for (int a = 0; a < NS; ++a) C[a] = rc * Y[a] / t.m.W[a];
+        net(T, C, wd);
+        double yy[NS];
+#pragma unroll
+        for (int a = 0; a < NS; ++a) {
+            drho[a] += dt / 2.0 * (double)u_rho_dot(A.U, (float)(wd[a] * t.m.W[a]));
+            yy[a] = (rho_a[a] + drho[a]) / rho;
+        }
+        set_mass_fractions<NS>(t, yy, Y, X);
+        rc = 1.0 / vol;
+        double Tn;
+        if (gas::T_from_u_n<NS>(t, Y, u_si, T, 1e-14, 100, Tn) < 0) atomic_status(A.status, LBMGPU_ST_NEWTON);
+        T = Tn;
+    }
+    double hrr = 0.0;
+#pragma unroll
+    for (int a = 0; a < NS; ++a) {
+        hrr += -1.0 * (double)u_energy_mass(A.U, (float)(gas::h_RT_q(t, a, T) * gas::kR * T / t.m.W[a])) * drho[a];
+        A.props[(long)pr_drho<NS>(a) * A.ncell + n] = drho[a];
+    }
+    put(A, A.rec_nxt, RM_HRR, n, hrr);
+}
+
+// The collision parameters of one cell.  CHEM: the chemistry to run with it (the host build; the
+// device runs the chemistry in kernels of its own, CHEM_OFF here).
 template <int NS, int CHEM, class AT>
 MC_HDN void mc_props_cell(const AT &A, long n) {
     const gas::Tables &t = *A.tab;
     const typename AT::R *Rc = A.rec_cur;
-    double *Pr = A.props;
-    auto prp = [&](int plane, double v) { Pr[(long)plane * A.ncell + n] = v; };
     const double rho = rec(A, Rc, RM_RHO, n);
-    const double um[3] = {rec(A, Rc, RM_U, n), rec(A, Rc, RM_V, n), rec(A, Rc, RM_W, n)};
-    const double Tl = rec(A, Rc, RM_T, n), p = rec(A, Rc, RM_P, n), rhoe = rec(A, Rc, RM_RHOE, n);
-    double rho_a[NS], ua[NS][3], Xs[NS];
-    for (int a = 0; a < NS; ++a) {
-        rho_a[a] = rec(A, Rc, rs(a, RS_RHO), n);
-        for (int d = 0; d < 3; ++d) ua[a][d] = rec(A, Rc, rs(a, RS_UX + d), n);
-        Xs[a] = rec(A, Rc, rs(a, RS_X), n);
-    }
-    // Cantera state (lbm-collision.cpp:364-367 and :236-238); the FP32 storage mode takes the
-    // reciprocal forms (rounding-level differences, as in its moment solve)
-    constexpr bool fast = sizeof(typename AT::P) == sizeof(float);
+    const double Tl = rec(A, Rc, RM_T, n), p = rec(A, Rc, RM_P, n);
+    double rho_a[NS];
+#pragma unroll
+    for (int a = 0; a < NS; ++a) rho_a[a] = rec(A, Rc, rs(a, RS_RHO), n);
     double Yr[NS], Y[NS], X[NS];
-    double W;
-    if constexpr (fast) {
-        const double ir = 1.0 / rho;
-        for (int a = 0; a < NS; ++a) Yr[a] = rho_a[a] * ir;
-        W = set_mass_fractions_fast<NS>(t, Yr, Y, X);
-    } else {
-        for (int a = 0; a < NS; ++a) Yr[a] = rho_a[a] / rho;
-        W = set_mass_fractions<NS>(t, Yr, Y, X);
-    }
+    const double W = mc_state<NS>(A, rho, rho_a, Yr, Y, X);
     const double T_si = si_temp(A.U, (float)Tl);
     const double rho_si = si_rho(A.U, (float)rho);
     const double P_si = rho_si * gas::kR * T_si / W;
-    const double dt = A.dt;
-
-    // internal energy without the species kinetic energy (lbm-collision.cpp:260-263, 373-376)
-    double Uint = rhoe / rho;
-    for (int a = 0; a < NS; ++a)
-        Uint = Uint - 0.5 * rho_a[a] / rho * (ua[a][0] * ua[a][0] + ua[a][1] * ua[a][1] + ua[a][2] * ua[a][2]);
-
-    // -- chemistry: two explicit half steps with T from (u, v) in between (lbm-collision.cpp:370-399)
+    const double Uint = mc_u_int<NS>(A, n, rho, Yr);
     if (CHEM == CHEM_REF_EXPLICIT) {
-        double drho[NS];
-        for (int a = 0; a < NS; ++a) drho[a] = 0.0;
-        double Tc = T_si, rc = rho_si, Yc[NS], Xc[NS];
-        for (int a = 0; a < NS; ++a) Yc[a] = Y[a];
-        for (int sub = 0; sub < 2; ++sub) {
-            double C[gas::MAXS], wd[gas::MAXS];
-            for (int a = 0; a < NS; ++a) C[a] = rc * Yc[a] / t.m.W[a];
-            gas::net_production(t, Tc, C, wd);
-            for (int a = 0; a < NS; ++a) drho[a] += dt / 2.0 * (double)u_rho_dot(A.U, (float)(wd[a] * t.m.W[a]));
-            double yy[NS];
-            for (int a = 0; a < NS; ++a) yy[a] = (rho_a[a] + drho[a]) / rho;
-            set_mass_fractions<NS>(t, yy, Yc, Xc);
-            const double vol = 1.0 / (double)si_rho(A.U, (float)rho);
-            rc = 1.0 / vol;
-            double Tn;
-            if (gas::T_from_u(t, Yc, si_energy_mass(A.U, (float)Uint), Tc, 1e-14, 100, Tn) < 0)
-                atomic_status(A.status, LBMGPU_ST_NEWTON);
-            Tc = Tn;
-        }
-        double hrr = 0.0;
-        for (int a = 0; a < NS; ++a) {
-            hrr += -1.0 * (double)u_energy_mass(A.U, (float)(gas::h_RT(t, a, Tc) * gas::kR * Tc / t.m.W[a])) * drho[a];
-            prp(pr_drho<NS>(a), drho[a]);
-        }
-        put(A, A.rec_nxt, RM_HRR, n, hrr);
-    } else if (CHEM == CHEM_ROSENBROCK) {  // the host build; the device runs it in k_mc_chem
+        mc_chem_explicit<NS>(A, n, gas::TableNet{t});
+    } else if (CHEM == CHEM_ROSENBROCK) {
         double rc, rac[NS], Yc[NS], Tc, rhoc, Pc;  // the state as k_mc_chem forms it
         mc_chem_state<NS>(A, n, rc, rac, Yc, Tc, rhoc, Pc);
         mc_chem_ros2<NS>(A, n, rc, rac, Yc, Tc, rhoc, Pc, true);
     }
-
     if constexpr (sizeof(typename AT::P) == sizeof(float))
-        mc_transport_f32<NS>(A, n, p, rho_a, ua, Xs, Y, X, W, T_si, P_si, Uint);
+        mc_transport_f32<NS>(A, n, p, rho_a, Y, X, W, T_si, P_si, Uint);
     else
-        mc_transport_f64<NS>(A, n, p, rho_a, ua, Xs, Y, X, W, T_si, P_si, Uint);
+        mc_transport_f64<NS>(A, n, p, rho_a, Y, X, W, T_si, P_si, Uint);
 }
 
 // The energy-flux terms of the energy collision (lbm-collision.cpp:265-316): the enthalpy

@@ -1,8 +1,8 @@
-// lbmgpu, multicomponent path: the stiff chemistry's kernels (LBMGPU_CHEM_ROSENBROCK: ROS2 of
-// every cell, the surrogate's use, the integrator list) and their launches, for one species
-// count NS.  They read the record and write the chemistry's collision parameters, no
-// populations, so one instance serves both population storages; a compilation unit of its own
-// (mc_chem<NS>.cu).
+// lbmgpu, multicomponent path: the chemistry's kernels and their launches, for one species count
+// NS, in a compilation unit of their own (mc_chem<NS>.cu): LBMGPU_CHEM_ROSENBROCK (ROS2 of every
+// cell, the surrogate's use, the integrator list) and LBMGPU_CHEM_REF_EXPLICIT.  They read the
+// record and write the chemistry's collision parameters, no populations; the stiff chemistry's
+// arithmetic does not depend on the population storage either, so one instance serves both.
 #pragma once
 #include <type_traits>
 
@@ -84,6 +84,21 @@ __global__ void __launch_bounds__(kBlock, SUR ? 4 : 2) k_mc_chem(McArgs A) {
     mc_chem_ros2<NS, McArgs, !SUR, 1, KIN, smat, PRED>(A, n, rho, rho_a, Y, T_si, rho_si, P_si, SUR);
 }
 
+// The reference's explicit chemistry of every fluid cell (mc_chem_explicit), one thread per cell.
+// NET: the net production rates -- the compiled kinetics of the handle's mechanism, or the dense
+// tables (gas::DenseNet).  A kernel of its own: inside the transport kernel the table-driven rates
+// (a RateT per temperature, 2.4 kB of local arrays) took 135 of 202 us at 512 cells and 180 of 248 us
+// at 33 k cells; here transport and chemistry together take 79 and 126 us.
+template <int NS, typename S, class NET>
+__global__ void __launch_bounds__(kBlock, 2) k_mc_explicit(McArgsT<S, double> A) {
+    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
+    if constexpr (std::is_same_v<NET, gas::DenseNet<NS>>)
+        mc_chem_explicit<NS>(A, n, NET{*A.tab});
+    else
+        mc_chem_explicit<NS>(A, n, NET{});
+}
+
 // The stiff chemistry over the compiled kinetics of the handle's mechanism, where the library
 // has them for it (kinetics_h2_air_9.cuh): every cell (k_mc_chem) or the integrator list
 // (k_mc_chem_list).  Returns false when the handle's mechanism is not compiled.
@@ -138,6 +153,21 @@ int chem_step(lbmgpu *h, const lbm::McArgs &A) {
         ev_end(h, ei);
         CK(cudaGetLastError());
     }
+    return 0;
+}
+
+template <int NS, typename S>
+int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A) {
+    const unsigned gp = grid_for(h->g.ncell);
+    bool compiled = false;
+    if constexpr (NS == kin_h2_air_9::NS) {
+        if (h->kin == KIN_H2_AIR_9) {
+            k_mc_explicit<NS, S, kin_h2_air_9::Kinetics><<<gp, kBlock, 0, h->stream>>>(A);
+            compiled = true;
+        }
+    }
+    if (!compiled) k_mc_explicit<NS, S, gas::DenseNet<NS>><<<gp, kBlock, 0, h->stream>>>(A);
+    CK(cudaGetLastError());
     return 0;
 }
 

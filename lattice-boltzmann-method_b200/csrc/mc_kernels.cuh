@@ -29,15 +29,17 @@ namespace {
 using namespace lbm;
 using namespace lbmh;
 
-// collision parameters of every fluid cell, one instance per chemistry mode; three blocks per
-// SM (168 registers).  FP32 storage: the transport runs in FP32 with its species loops
-// unrolled, so its per-species arrays live in registers (at 128 registers, four blocks per SM,
-// they spilled: 2.00 ms against 1.21 ms at 128^3)
-template <int NS, int CHEM, typename S>
+// Transport part of the collision parameters of every fluid cell (the chemistry runs in kernels of
+// its own, mc_chem.cuh), one thread per cell.  Bound by the latency of its FP64 chains and of the record
+// loads, not by HBM; three blocks per SM (168 registers), the species loops unrolled, so the
+// per-species arrays live in registers, the species velocities loaded where the Maxwell-Stefan force
+// uses them.  FP64 storage, 48 x 40 x 37 cells: 189 us with rolled loops (920 B of local arrays) and
+// 400 divisions per cell, 119 us now; FP32 storage, 96^3: 523 -> 502 us.
+template <int NS, typename S>
 __global__ void __launch_bounds__(kBlock, 3) k_mc_props(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
-    mc_props_cell<NS, CHEM>(A, n);
+    mc_props_cell<NS, CHEM_OFF>(A, n);
 }
 
 // The energy-flux terms of the collision (mc_eflux_cell), after the collision parameters.
@@ -308,10 +310,11 @@ int collide_t(lbmgpu *h) {
     EvPair ep{};
     ev_begin(h, K_PROPS, ep);
     const unsigned gp = grid_for(h->g.ncell);
-    if (h->chem == CHEM_REF_EXPLICIT)
-        k_mc_props<NS, CHEM_REF_EXPLICIT, S><<<gp, kBlock, 0, h->stream>>>(A);
-    else
-        k_mc_props<NS, CHEM_OFF, S><<<gp, kBlock, 0, h->stream>>>(A);  // ROS2 / surrogate: k_mc_chem
+    k_mc_props<NS, S><<<gp, kBlock, 0, h->stream>>>(A);
+    if (h->chem == CHEM_REF_EXPLICIT) {
+        const int rc_ = explicit_step<NS, S>(h, A);
+        if (rc_) return rc_;
+    }
     ev_end(h, ep);
     CK(cudaGetLastError());
     if (h->chem == CHEM_ROSENBROCK) {

@@ -69,9 +69,15 @@ struct McOps {
     static constexpr int props_planes() { return lbm::pr_count<NS>(); }
     static constexpr int gsum_planes() { return lbm::gs_count<NS>(); }
 };
-// The stiff chemistry of one collision (mc_chem.cuh, instantiated in mc_chem<NS>.cu).
+// The chemistry of one collision, stiff and explicit (mc_chem.cuh, instantiated in mc_chem<NS>.cu).
 template <int NS>
 int chem_step(lbmgpu *h, const lbm::McArgs &A);
+template <int NS, typename S>
+int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A);
+extern template int explicit_step<9, double>(lbmgpu *, const lbm::McArgsT<double, double> &);
+extern template int explicit_step<9, float>(lbmgpu *, const lbm::McArgsT<float, double> &);
+extern template int explicit_step<6, double>(lbmgpu *, const lbm::McArgsT<double, double> &);
+extern template int explicit_step<6, float>(lbmgpu *, const lbm::McArgsT<float, double> &);
 extern template int chem_step<9>(lbmgpu *, const lbm::McArgs &);
 extern template int chem_step<6>(lbmgpu *, const lbm::McArgs &);
 // The boundary cells of one streaming on the side stream (mc_special.cuh, instantiated in

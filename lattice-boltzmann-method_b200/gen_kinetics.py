@@ -587,6 +587,28 @@ def generate(m, name):
     emit_rhs_epilogue(m, add)
     add("}")
     add("")
+    # ---- net production rates
+    add("// Net molar production rates w [kmol/m^3/s] at temperature T and concentrations C [kmol/m^3], from")
+    add("// the thermo th at T (gas::net_production, reaction by reaction).")
+    add("GAS_HD void net_t(const Thermo &th, double T, const double *C, double *w) {")
+    add("    const double logT = th.logT, invRT = th.invRT, log_cref = th.log_cref;")
+    add("    (void)T;")
+    add("    (void)logT;")
+    add("    (void)log_cref;")
+    for k in range(m.n_species):
+        add(f"    const double C{k} = C[{k}];")
+    for k in range(m.n_species):
+        add(f"    double w{k} = 0.0;")
+    for r in range(nr):
+        add("    GAS_SCHED_FENCE();")
+        add(f"    {{  // reaction {r}")
+        emit_rates(m, r, fidx, add, N)
+        emit_rhs_reaction(m, r, fidx, add, N, names)
+        add("    }")
+    for k in range(m.n_species):
+        add(f"    w[{k}] = w{k};")
+    add("}")
+    add("")
     # ---- right-hand side and Jacobian together
     _, comps = system_index(m)
     inert = inert_species(m)
@@ -627,6 +649,12 @@ def generate(m, name):
     add(f"    GAS_HD static constexpr int sys_full(int i) {{ return {chain}; }}")
     add("    GAS_HD void factors(double T, Thermo &k) const { thermo(T, k); }")
     add("    GAS_HD void rhs(const Thermo &k, double rho, const double *y, double *F) const { rhs_t(k, rho, y, F); }")
+    add("    // net production rates at (T, C): the explicit scheme's policy")
+    add("    GAS_HD void operator()(double T, const double *C, double *w) const {")
+    add("        Thermo th;")
+    add("        thermo(T, th);")
+    add("        net_t(th, T, C, w);")
+    add("    }")
     add("    template <class Mat>")
     add("    GAS_HD void rhs_jacobian(const Thermo &k, double rho, const double *y, double *F, double s, Mat &J) const {")
     add("        rhs_jac(k, rho, y, F, s, J);")
