@@ -59,6 +59,16 @@ __global__ void __launch_bounds__(kMeanBlock) k_plane_mean(McArgsT<S, double> A,
     if (threadIdx.x == 0) shift_new[q] = nfluid > 0 ? red[0] / (double)nfluid : 0.0;
 }
 
+// the shift's own momentum per set, sum_l shift c_l, behind the planes' shifts (k_mc_relax)
+__global__ void k_shift_sums(double *shift, int nset) {
+    const int i = threadIdx.x;
+    if (i >= 3 * nset) return;
+    const int a = i / 3, d = i % 3;
+    double s = 0.0;
+    for (int l = 0; l < 27; ++l) s += shift[27 * a + l] * (d == 0 ? cx(l) : (d == 1 ? cy(l) : cz(l)));
+    shift[27 * nset + i] = s;
+}
+
 // ... and both population buffers re-encoded from the old shift to the new one.
 template <typename S>
 __global__ void k_reshift(long total, long ncell, S *p0, S *p1, const double *old_s, const double *new_s) {
@@ -102,6 +112,8 @@ int rebase_shift(lbmgpu *h) {
     McArgsT<float, double> A = base_args<float>(h);
     const int np = 27 * (h->ns + 1);
     k_plane_mean<float><<<np, kMeanBlock, 0, h->stream>>>(A, h->pop32[h->cur], h->shift[1], h->nfluid);
+    CK(cudaGetLastError());
+    k_shift_sums<<<1, 64, 0, h->stream>>>(h->shift[1], h->ns + 1);
     CK(cudaGetLastError());
     const long total = (long)np * h->g.ncell;
     k_reshift<float><<<grid_for(total), kBlock, 0, h->stream>>>(total, h->g.ncell, h->pop32[0], h->pop32[1],
@@ -150,9 +162,10 @@ int mc_setup(lbmgpu *h) {
         CK(cudaMemset(h->fp32 ? (void *)h->pop32[b] : (void *)h->pop[b], 0,
                       np * nc * (h->fp32 ? sizeof(float) : sizeof(double))));
         if (h->fp32) {
-            rc = dalloc(h, &h->shift[b], np);
+            const size_t nsh = np + 3 * (size_t)(h->ns + 1);  // the planes' shifts, then each set's momentum
+            rc = dalloc(h, &h->shift[b], nsh);
             if (rc) return rc;
-            CK(cudaMemset(h->shift[b], 0, np * sizeof(double)));
+            CK(cudaMemset(h->shift[b], 0, nsh * sizeof(double)));
         }
     }
     h->kin = kin_h2_air_9::matches(*d.mech) ? KIN_H2_AIR_9 : KIN_TABLES;

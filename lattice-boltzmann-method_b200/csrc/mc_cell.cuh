@@ -179,9 +179,7 @@ struct McPull {
     long X[3], Y[3], Z[3];
 };
 template <class AT>
-MC_HD void mc_pull(const AT &A, long n, McPull &p) {
-    int i, j, k;
-    cell_ijk(n, A.si, A.sj, i, j, k);
+MC_HD void mc_pull(const AT &A, int i, int j, int k, McPull &p) {
     const int im = (i - 1 == 0 && !A.halo_lo) ? A.Nx - 2 : i - 1;
     const int ip = (i + 1 == A.Nx - 1 && !A.halo_hi) ? 1 : i + 1;
     const int jm = (j - 1 == 0) ? A.Ny - 2 : j - 1, jp = (j + 1 == A.Ny - 1) ? 1 : j + 1;
@@ -195,6 +193,12 @@ MC_HD void mc_pull(const AT &A, long n, McPull &p) {
     p.Z[0] = k;
     p.Z[1] = km;
     p.Z[2] = kp;
+}
+template <class AT>
+MC_HD void mc_pull(const AT &A, long n, McPull &p) {
+    int i, j, k;
+    cell_ijk(n, A.si, A.sj, i, j, k);
+    mc_pull(A, i, j, k, p);
 }
 MC_HD long pull_idx(const McPull &p, int l) { return p.X[cidx(cx(l))] + p.Y[cidx(cy(l))] + p.Z[cidx(cz(l))]; }
 

@@ -22,6 +22,7 @@
 #include "mc_bc.cuh"
 #include "mc_cell.cuh"
 #include "mc_ops.cuh"
+#include "mc_relax.cuh"
 #include "surrogate_host.cuh"
 
 namespace {
@@ -48,19 +49,6 @@ __global__ void __launch_bounds__(kBlock) k_mc_eflux(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
     mc_eflux_cell<NS>(A, n);
-}
-
-// BGK update: blockIdx.y selects the population set (species 0..NS-1, NS = energy), the
-// x dimension the cells, so a warp reads one set's planes at 32 consecutive cells
-template <int NS, typename S>
-__global__ void __launch_bounds__(kBlock, 4) k_mc_relax(McArgsT<S, double> A) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
-    const int a = blockIdx.y;
-    if (a < NS)
-        mc_relax_species<NS>(A, n, a);
-    else
-        mc_relax_energy<NS>(A, n);
 }
 
 // Interior cells (no boundary upstream): the pull of one population set per thread
@@ -332,7 +320,11 @@ int collide_t(lbmgpu *h) {
     CK(cudaGetLastError());
     EvPair er{};
     ev_begin(h, K_COLLIDE, er);
-    k_mc_relax<NS, S><<<dim3(grid_for(h->g.ncell), NS + 1), kBlock, 0, h->stream>>>(A);
+    const dim3 gr(grid_for(h->g.ncell), NS + 1);
+    if (h->chem == CHEM_OFF)
+        k_mc_relax<NS, false, S><<<gr, kBlock, 0, h->stream>>>(A);
+    else
+        k_mc_relax<NS, true, S><<<gr, kBlock, 0, h->stream>>>(A);
     ev_end(h, er);
     CK(cudaGetLastError());
     return 0;
