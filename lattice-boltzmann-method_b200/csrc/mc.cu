@@ -59,14 +59,11 @@ __global__ void __launch_bounds__(kMeanBlock) k_plane_mean(McArgsT<S, double> A,
     if (threadIdx.x == 0) shift_new[q] = nfluid > 0 ? red[0] / (double)nfluid : 0.0;
 }
 
-// the shift's own momentum per set, sum_l shift c_l, behind the planes' shifts (k_mc_relax)
+// the shift's own sums per set (species_sums of its 27 values) behind the planes' shifts: the kernels
+// that sum or relax stored deviations add them (k_mc_gather, k_mc_relax)
 __global__ void k_shift_sums(double *shift, int nset) {
-    const int i = threadIdx.x;
-    if (i >= 3 * nset) return;
-    const int a = i / 3, d = i % 3;
-    double s = 0.0;
-    for (int l = 0; l < 27; ++l) s += shift[27 * a + l] * (d == 0 ? cx(l) : (d == 1 ? cy(l) : cz(l)));
-    shift[27 * nset + i] = s;
+    const int a = threadIdx.x;
+    if (a < nset) species_sums(shift + 27 * a, shift + 27 * nset + kGsPerSpecies * a);
 }
 
 // ... and both population buffers re-encoded from the old shift to the new one.
@@ -113,7 +110,7 @@ int rebase_shift(lbmgpu *h) {
     const int np = 27 * (h->ns + 1);
     k_plane_mean<float><<<np, kMeanBlock, 0, h->stream>>>(A, h->pop32[h->cur], h->shift[1], h->nfluid);
     CK(cudaGetLastError());
-    k_shift_sums<<<1, 64, 0, h->stream>>>(h->shift[1], h->ns + 1);
+    k_shift_sums<<<1, 32, 0, h->stream>>>(h->shift[1], h->ns + 1);
     CK(cudaGetLastError());
     const long total = (long)np * h->g.ncell;
     k_reshift<float><<<grid_for(total), kBlock, 0, h->stream>>>(total, h->g.ncell, h->pop32[0], h->pop32[1],
@@ -152,8 +149,6 @@ int mc_setup(lbmgpu *h) {
         if (b == 0) {
             rc = dalloc(h, &h->props, (size_t)mc_by_ns(h->ns, [](auto ops) { return decltype(ops)::props_planes(); }) * nc);
             if (rc) return rc;
-            rc = dalloc(h, &h->gsum, (size_t)mc_by_ns(h->ns, [](auto ops) { return decltype(ops)::gsum_planes(); }) * nc);
-            if (rc) return rc;
         }
         // the face-difference planes of cells the kernels never write (ghosts) are read
         // but not used, and the ghosts' populations are never read; zero them all so they
@@ -162,7 +157,7 @@ int mc_setup(lbmgpu *h) {
         CK(cudaMemset(h->fp32 ? (void *)h->pop32[b] : (void *)h->pop[b], 0,
                       np * nc * (h->fp32 ? sizeof(float) : sizeof(double))));
         if (h->fp32) {
-            const size_t nsh = np + 3 * (size_t)(h->ns + 1);  // the planes' shifts, then each set's momentum
+            const size_t nsh = np + kGsPerSpecies * (size_t)(h->ns + 1);  // the planes' shifts, then each set's sums
             rc = dalloc(h, &h->shift[b], nsh);
             if (rc) return rc;
             CK(cudaMemset(h->shift[b], 0, nsh * sizeof(double)));
@@ -187,8 +182,6 @@ void mc_release(lbmgpu *h) {
     h->tab = nullptr;
     cudaFree(h->props);
     h->props = nullptr;
-    cudaFree(h->gsum);
-    h->gsum = nullptr;
     for (int b = 0; b < 2; ++b) {
         cudaFree(h->pop32[b]);
         cudaFree(h->bst32[b]);

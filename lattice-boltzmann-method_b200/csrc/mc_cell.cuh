@@ -301,14 +301,12 @@ template <int NS> MC_HD constexpr int pr_count() { return pr_gc<NS>() + 1; }
 // species: rho_a, j_a and its share of the P tensor; the energy set's sum), then the
 // per-cell solve from the sums (Stefan-Maxwell species velocities, temperature, record).
 // The P tensor is summed species by species (each species' share over its 27 directions,
-// then the shares in species order) on every path, so the interior split into a gather
-// kernel and a solve kernel gives the same bits as the one-pass function.
+// then the shares in species order) on every path, so the interior's kernels (mc_moments.cuh) and
+// this function add the same terms in the same order.
 // ------------------------------------------------------------------------------------
 constexpr int kGsPerSpecies = 10;  // rho_a, j_a (3), P-tensor share (6)
-template <int NS> MC_HD constexpr int gs_count() { return kGsPerSpecies * NS + 1; }
 
-// The sums of one cell held in registers (the one-pass path); SumsAt reads the same
-// values from the gathered planes where they are used.
+// The sums of one cell.
 template <int NS>
 struct McSums {
     double ra[NS], ja[NS][3], p6[6], re;
@@ -340,23 +338,6 @@ MC_HD void species_sums(const double *fv, double *s) {
     s[3] = jz;
     for (int q = 0; q < 6; ++q) s[4 + q] = p[q];
 }
-
-// The gathered sum planes of cell n (k_mc_gather): species a at planes 10a..10a+9, the
-// energy sum at 10 NS; the P tensor adds the species' shares in species order.
-template <int NS>
-struct SumsAt {
-    const double *gs;
-    long ncell, n;
-    MC_HD double at(int plane) const { return gs[(long)plane * ncell + n]; }
-    MC_HD double rho_a(int a) const { return at(kGsPerSpecies * a); }
-    MC_HD double j(int a, int d) const { return at(kGsPerSpecies * a + 1 + d); }
-    MC_HD double P6(int q) const {
-        double v = 0.0;
-        for (int a = 0; a < NS; ++a) v += at(kGsPerSpecies * a + 4 + q);
-        return v;
-    }
-    MC_HD double rhoe() const { return at(kGsPerSpecies * NS); }
-};
 
 template <int NS, class AT, class Sums>
 MC_HDN void mc_moments_finish(const AT &A, long n, const Sums &S);

@@ -6,8 +6,8 @@
 //   LBM::Collide_Species + LBM::Collide   src/lbm-collision.cpp:191-526 -> k_mc_props, the stiff
 //                                          chemistry (mc_chem.cuh), k_mc_eflux, k_mc_relax
 //   LBM::Streaming + LBM::calculate_moment src/lbm-streaming.cpp, src/lbm-moment.cpp:193-377
-//                                          -> k_mc_gather (pull + population sums per
-//                                             (cell, set)) and k_mc_solve (per cell)
+//                                          -> k_mc_gather (pull + population sums),
+//                                             k_mc_diffuse and k_mc_thermo (mc_moments.cuh)
 //   LBM::Init                              src/lbm-init.cpp:85-146 -> k_mc_init
 //   LBM::Streaming + LBM::TMS_BC + LBM::calculate_moment of the cells with a boundary
 //   upstream (src/lbm-bc.cpp:122-1110, src/impose_nscbc.cpp) -> k_mc_special (mc_special.cuh)
@@ -21,6 +21,7 @@
 #include "handle.cuh"
 #include "mc_bc.cuh"
 #include "mc_cell.cuh"
+#include "mc_moments.cuh"
 #include "mc_ops.cuh"
 #include "mc_relax.cuh"
 #include "surrogate_host.cuh"
@@ -49,42 +50,6 @@ __global__ void __launch_bounds__(kBlock) k_mc_eflux(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
     mc_eflux_cell<NS>(A, n);
-}
-
-// Interior cells (no boundary upstream): the pull of one population set per thread
-// (blockIdx.y = species, NS = the energy set) and its sums into the gsum planes --
-// species a: rho_a, j_a, its P-tensor share at planes 10a..10a+9; the energy set's sum at
-// plane 10 NS.  A warp reads one set's planes at 32 consecutive cells.
-template <int NS, typename S>
-__global__ void __launch_bounds__(kBlock, 4) k_mc_gather(McArgsT<S, double> A, double *__restrict__ gs) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= A.ncell || A.cflag[n] != CF_FLUID) return;
-    const int a = blockIdx.y;
-    McPull pp;
-    mc_pull(A, n, pp);
-    if (a < NS) {
-        double fv[27], s[kGsPerSpecies];
-#pragma unroll
-        for (int l = 0; l < 27; ++l) fv[l] = ldpop(A, A.pop_src, 27 * a + l, pull_idx(pp, l));
-        species_sums(fv, s);
-#pragma unroll
-        for (int q = 0; q < kGsPerSpecies; ++q) gs[(long)(kGsPerSpecies * a + q) * A.ncell + n] = s[q];
-    } else {
-        double e = 0.0;
-#pragma unroll
-        for (int l = 0; l < 27; ++l) e += ldpop(A, A.pop_src, 27 * NS + l, pull_idx(pp, l));
-        gs[(long)(kGsPerSpecies * NS) * A.ncell + n] = e;
-    }
-}
-
-// Interior cells: the moment solve from the gathered sums (species velocities from the
-// Stefan-Maxwell system, temperature, the record) -- the same bits as mc_stream_moment_cell.
-template <int NS, typename S>
-__global__ void __launch_bounds__(kBlock, 2) k_mc_solve(McArgsT<S, double> A, const double *__restrict__ gs) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= A.ncell || A.cflag[n] != CF_FLUID) return;
-    const SumsAt<NS> Sm{gs, A.ncell, n};
-    mc_moments_finish<NS>(A, n, Sm);
 }
 
 template <int NS, typename S>
@@ -353,12 +318,13 @@ int stream_t(lbmgpu *h) {
     }
     EvPair ep{};
     ev_begin(h, K_STREAM_MOMENT, ep);
-    k_mc_gather<NS, S><<<dim3(grid_for(h->g.ncell), NS + 1), kBlock, 0, h->stream>>>(A, h->gsum);
+    k_mc_gather<NS, S><<<(unsigned)((h->g.ncell + kGatherCells - 1) / kGatherCells), kGatherCells *(NS + 1), 0, h->stream>>>(A);
     ev_end(h, ep);
     CK(cudaGetLastError());
     EvPair es{};
     ev_begin(h, K_SOLVE, es);
-    k_mc_solve<NS, S><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(A, h->gsum);
+    k_mc_diffuse<NS, S><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(A);
+    k_mc_thermo<NS, S><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(A);
     ev_end(h, es);
     CK(cudaGetLastError());
     if (h->nb > 0) CK(cudaStreamWaitEvent(h->stream, h->join, 0));

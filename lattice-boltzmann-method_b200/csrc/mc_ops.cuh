@@ -67,7 +67,6 @@ struct McOps {
     static int stream(lbmgpu *h);
     static int halo(lbmgpu *h, int face, int what, double *buf, bool pack);
     static constexpr int props_planes() { return lbm::pr_count<NS>(); }
-    static constexpr int gsum_planes() { return lbm::gs_count<NS>(); }
 };
 // The chemistry of one collision, stiff and explicit (mc_chem.cuh, instantiated in mc_chem<NS>.cu).
 template <int NS>

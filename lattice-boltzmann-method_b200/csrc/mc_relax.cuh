@@ -23,6 +23,7 @@
 // bytes cost more issue slots than the latency they hide.
 #pragma once
 #include "mc_cell.cuh"
+#include "mc_moments.cuh"
 
 namespace lbm {
 
@@ -41,28 +42,6 @@ static_assert(dir3_ok(), "dir3 inverts cx, cy, cz");
 // Blocks of 128 threads per SM.  Five (96 registers) spill 340 B: 971 for 975 us in FP32, 111 for
 // 104 us in FP64.
 constexpr int kRelaxBlocks = 4;
-
-// The cell of the interior nearest to n: itself for every fluid cell.  A thread loads what cell n
-// will need at this cell before it knows whether n is a fluid cell at all, so that the flag's load and
-// the values' loads are one round of memory latency instead of two.
-template <class AT>
-__device__ __forceinline__ long interior_pull(const AT &A, long n, unsigned (&X)[3], unsigned (&Y)[3], unsigned (&Z)[3]) {
-    int i, j, k;
-    cell_ijk(n, A.si, A.sj, i, j, k);
-    i = min(max(i, 1), A.Nx - 2);
-    j = min(max(j, 1), A.Ny - 2);
-    k = min(max(k, 1), A.Nz - 2);
-    const long m = (long)i * A.si + (long)j * A.sj + k;
-    McPull pp;
-    mc_pull(A, i, j, k, pp);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        X[c] = (unsigned)pp.X[c];
-        Y[c] = (unsigned)pp.Y[c];
-        Z[c] = (unsigned)pp.Z[c];
-    }
-    return m;
-}
 
 // The 27 stored populations of set a: pulled to interior cell m, or (local mode) in place.
 template <class AT>
@@ -255,7 +234,7 @@ __global__ void __launch_bounds__(128, kRelaxBlocks) k_mc_relax(McArgsT<S, doubl
     const int a = blockIdx.y;
     __shared__ double sh[30];  // FP32 storage: the set's 27 shifts and their momentum
     if (sizeof(S) == sizeof(float) && threadIdx.x < 30)
-        sh[threadIdx.x] = A.shift[threadIdx.x < 27 ? 27 * a + threadIdx.x : 27 * (NS + 1) + 3 * a + threadIdx.x - 27];
+        sh[threadIdx.x] = A.shift[threadIdx.x < 27 ? 27 * a + threadIdx.x : 27 * (NS + 1) + kGsPerSpecies * a + 1 + threadIdx.x - 27];
     if (a < NS)
         relax_species_dev<NS, CHEM>(A, n, n < A.ncell, a, sh, sh + 27);
     else
