@@ -21,6 +21,7 @@
 #include "handle.cuh"
 #include "mc_bc.cuh"
 #include "mc_cell.cuh"
+#include "mc_eflux.cuh"
 #include "mc_moments.cuh"
 #include "mc_ops.cuh"
 #include "mc_relax.cuh"
@@ -42,14 +43,6 @@ __global__ void __launch_bounds__(kBlock, 3) k_mc_props(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
     mc_props_cell<NS, CHEM_OFF>(A, n);
-}
-
-// The energy-flux terms of the collision (mc_eflux_cell), after the collision parameters.
-template <int NS, typename S>
-__global__ void __launch_bounds__(kBlock) k_mc_eflux(McArgsT<S, double> A) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
-    mc_eflux_cell<NS>(A, n);
 }
 
 template <int NS, typename S>
