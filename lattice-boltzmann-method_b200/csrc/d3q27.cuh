@@ -51,6 +51,18 @@ __host__ __device__ constexpr int opp(int l) { return l == 0 ? 0 : ((l & 1) ? l 
 // index 0,1,2 of the per-axis factor tables for c = 0, +1, -1
 __host__ __device__ constexpr int cidx(int c) { return c == 0 ? 0 : (c == 1 ? 1 : 2); }
 
+// direction of the axis indices (0, 1, 2 for c = 0, +1, -1)
+__host__ __device__ constexpr int dir3(int ix, int iy, int iz) {
+    constexpr int8_t t[27] = {0, 5, 6, 3, 11, 17, 4, 18, 12, 1, 9, 15, 7, 19, 21, 13, 23, 26, 2, 16, 10, 14, 25, 24, 8, 22, 20};
+    return t[9 * ix + 3 * iy + iz];
+}
+constexpr bool dir3_ok() {
+    for (int l = 0; l < 27; ++l)
+        if (dir3(cidx(cx(l)), cidx(cy(l)), cidx(cz(l))) != l) return false;
+    return true;
+}
+static_assert(dir3_ok(), "dir3 inverts cx, cy, cz");
+
 // Per-axis factors of the product-form equilibrium (reference calculate_feq,
 // src/headers/lbm.hpp:276-305): psi_0 = 1 - zeta, psi_+-1 = (+-xi + zeta)/2.
 template <typename R>

@@ -20,6 +20,7 @@
 #include "handle.cuh"
 #include "mc_ops.cuh"
 #include "sc_kernels.cuh"
+#include "sc_special.cuh"
 #include "sums.cuh"
 #include "halo.cuh"
 
@@ -50,33 +51,54 @@ __device__ __forceinline__ double fd_central(double sl, double sc, double sr, in
 // streams through the 27 directions: fetch f_l, g_l (pulled from the last collision's
 // output, or the special-cell store, or -- in local mode -- in place), relax, store.
 // ----------------------------------------------------------------------------------
-// Population q (0..53: f then g) of cell n at the start of the collision: in place
-// (local mode), from the special-cell store, or pulled from the upstream cell.
-__device__ __forceinline__ double fetch_pop(const double *__restrict__ src, const double *__restrict__ bst, long nc,
-                                            long nb, long n, long b, const PullSrc &ps, int q, bool local,
-                                            bool special) {
-    if (local) return src[(long)q * nc + n];
-    if (special) return bst[(long)q * nb + b];
-    return src[(long)q * nc + pull_at(ps, q % 27)];
-}
-
+//
+// A block takes 128 cells with 256 threads: half 0 relaxes f, half 1 relaxes g.  Each thread issues
+// everything it needs -- its 27 populations, the record, the face terms and types -- before its
+// cell's flag is known (at the nearest interior cell), so a block waits for one round of memory
+// latency; one thread for both sets went through four (flag, record, f, g).
+// Measured: 150 x 121 x 113 cells 440 -> 349 us (970 B a cell: 5.7 TB/s), 64^3 68 -> 52 us.
 template <bool LOCAL>
-__global__ void __launch_bounds__(kBlock, 4)
+__global__ void __launch_bounds__(2 * kBlock, 2)
     k_sc_collide(ScGeom g, ScPhys P, const int8_t *__restrict__ type, const uint8_t *__restrict__ cflag,
                  const int *__restrict__ bid, const double *__restrict__ src, double *__restrict__ dst,
                  const double *__restrict__ mom, const double *__restrict__ bst, long nb, unsigned *status) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= g.ncell) return;
+    const int set = threadIdx.x / kBlock;  // 0: f, 1: g
+    const long n = (long)blockIdx.x * kBlock + threadIdx.x % kBlock, nc = g.ncell;
+    if (n >= nc) return;
     const uint8_t cf = cflag[n];
+    PullSrc ps;
+    const long m = pull_interior(g, n, ps);
+    const double *const s0 = src + (long)27 * set * nc;
+    double v[27];
+#pragma unroll
+    for (int l = 0; l < 27; ++l) v[l] = (s0 + (long)l * nc)[LOCAL ? (unsigned)m : (unsigned)pull_at(ps, l)];
+    auto rec = [&](int q) { return mom[(long)q * nc + m]; };
+    const double rho = rec(M_RHO), T = rec(M_T), p = rec(M_P);
+    const double vel[3] = {rec(M_U), rec(M_V), rec(M_W)};
+    double q[3][3];
+    int tl[3], th[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const long off = a == 0 ? g.si : (a == 1 ? g.sj : 1);
+        const double *const Q = mom + (long)(M_QX + a) * nc + m;
+        q[a][0] = *(Q - off);
+        q[a][1] = *Q;
+        q[a][2] = Q[off];
+        tl[a] = type[m - off];
+        th[a] = type[m + off];
+    }
+    double S[3] = {0.0, 0.0, 0.0}, Uint = 0.0;
+    if (set == 1) {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) S[a] = rec(M_SX + a);
+        Uint = rec(M_UINT);
+    }
     if (!(cf & CF_FLUID)) return;
-    const long nc = g.ncell;
-
-    const double rho = mom[M_RHO * nc + n];
-    const double vel[3] = {mom[M_U * nc + n], mom[M_V * nc + n], mom[M_W * nc + n]};
-    const double T = mom[M_T * nc + n];
-    const double p = mom[M_P * nc + n];
-    const double S[3] = {mom[M_SX * nc + n], mom[M_SY * nc + n], mom[M_SZ * nc + n]};
-    const double Uint = mom[M_UINT * nc + n];
+    if (!LOCAL && (cf & CF_SPECIAL)) {
+        const double *const b0 = bst + (long)27 * set * nb + bid[n];
+#pragma unroll
+        for (int l = 0; l < 27; ++l) v[l] = b0[(long)l * nb];
+    }
 
     const double dt = P.dt;
     const double theta = P.R * T;
@@ -84,88 +106,59 @@ __global__ void __launch_bounds__(kBlock, 4)
     const double kappa = mu * P.cp / P.prtl;
     const double om1 = 2 * p * P.cp * dt / (p * P.cp * dt + 2 * kappa);
     const double om = 2 * p * dt / (p * dt + 2 * mu);
-    if (!(1.0 / om > 0.5) || !(1.0 / om1 > 0.5)) raise_status(status, LBMGPU_ST_TAU_UNSTABLE);
-
-    double dq[3], corr[3];
+    double dQ[3];
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const long off = a == 0 ? g.si : (a == 1 ? g.sj : 1);
-        const long nlo = n - off, nhi = n + off;
-        const double *Q = mom + (long)(M_QX + a) * nc;
-        const double dQ = fd_central(Q[nlo], Q[n], Q[nhi], type[nlo], type[nhi]);
-        dq[a] = S[a] + 0.5 * dt * vel[a] * dQ;
-        corr[a] = dt * (2 - om) / (2 * rho * om) * dQ;
+    for (int a = 0; a < 3; ++a) dQ[a] = fd_central(q[a][0], q[a][1], q[a][2], tl[a], th[a]);
+    double *const d0 = dst + (long)27 * set * nc + n;
+    if (set == 0) {
+        if (!(1.0 / om > 0.5) || !(1.0 / om1 > 0.5)) raise_status(status, LBMGPU_ST_TAU_UNSTABLE);
+        double corr[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) corr[a] = dt * (2 - om) / (2 * rho * om) * dQ[a];
+        AxisF<double> F;
+        axis_feq(F, vel, theta, corr);
+#pragma unroll
+        for (int l = 0; l < 27; ++l) d0[(long)l * nc] = (1.0 - om) * v[l] + om * feq_l(l, rho, F);
+        return;
     }
-    AxisF<double> F;
-    axis_feq(F, vel, theta, corr);
+    double dq[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) dq[a] = S[a] + 0.5 * dt * vel[a] * dQ[a];
     AxisG<double> G;
     axis_geq(G, Uint, theta, vel);
-
-    const bool special = cf & CF_SPECIAL;
-    PullSrc ps;
-    if (!LOCAL && !special) pull_src(g, n, ps);
-    const long b = special ? (long)bid[n] : 0;
-    // Each population set is fetched with all 27 loads issued back to back before any is
-    // used (the kernel is bound by memory latency; this keeps 27 loads in flight per
-    // thread), then relaxed and stored.
-    double v[27];
-#pragma unroll
-    for (int l = 0; l < 27; ++l) v[l] = fetch_pop(src, bst, nc, nb, n, b, ps, l, LOCAL, special);
-#pragma unroll
-    for (int l = 0; l < 27; ++l) dst[(long)l * nc + n] = (1.0 - om) * v[l] + om * feq_l(l, rho, F);
-#pragma unroll
-    for (int l = 0; l < 27; ++l) v[l] = fetch_pop(src, bst, nc, nb, n, b, ps, 27 + l, LOCAL, special);
+    const double kq = 0.5 * (om1 - om);
 #pragma unroll
     for (int l = 0; l < 27; ++l) {
         const double gq = geq_l(l, rho, G);
-        const double gs = (csq(l) == 1) ? gq + 0.5 * (cx(l) * dq[0] + cy(l) * dq[1] + cz(l) * dq[2]) : gq;
-        dst[(long)(27 + l) * nc + n] = v[l] + om1 * (gq - v[l]) + (om - om1) * (gq - gs);
+        double out = v[l] + om1 * (gq - v[l]);
+        if (csq(l) == 1)  // the flux correction acts along the six axes
+            out += kq * (cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2]));
+        d0[(long)l * nc] = out;
     }
 }
 
 // ----------------------------------------------------------------------------------
 // Streaming + moments for the cells with no boundary neighbour (reference LBM::Streaming
 // and LBM::calculate_moment, src/lbm-streaming.cpp:88-117, src/lbm-moment.cpp:11-125).
+// Bound by HBM on large lattices (536 B per cell); the loads are issued before the flag is known.
 // ----------------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock, 4)
     k_sc_stream_moment(ScGeom g, ScPhys P, const uint8_t *__restrict__ cflag, const double *__restrict__ src,
                        double *__restrict__ mom_nxt, unsigned *status) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= g.ncell) return;
-    if (cflag[n] != CF_FLUID) return;  // not fluid, or special (k_sc_stream_moment_special)
+    const uint8_t cf = cflag[n];
     const long nc = g.ncell;
     PullSrc ps;
-    pull_src(g, n, ps);
+    pull_interior(g, n, ps);
     ScSums s;
     sums_init(s);
 #pragma unroll
     for (int l = 0; l < 27; ++l) {
-        const long sidx = pull_at(ps, l);
-        sums_add(s, l, src[(long)l * nc + sidx], src[(long)(27 + l) * nc + sidx]);
+        const unsigned sidx = (unsigned)pull_at(ps, l);
+        sums_add(s, l, (src + (long)l * nc)[sidx], (src + (long)(27 + l) * nc)[sidx]);
     }
-    store_record_sc(g, P, n, s, mom_nxt, status);
-}
-
-// The same for the special cells (compact list): streaming with bounce-back, free-slip
-// and persisting populations, the TMS boundary treatment (reference LBM::TMS_BC), moments.
-__global__ void __launch_bounds__(kBlock)
-    k_sc_stream_moment_special(ScGeom g, ScPhys P, const int8_t *__restrict__ type, const long *__restrict__ blist,
-                               const double *__restrict__ src, const double *__restrict__ mom_cur,
-                               double *__restrict__ mom_nxt, const double *__restrict__ bst_cur,
-                               double *__restrict__ bst_nxt, long nb, unsigned *status) {
-    const long b = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const long n = blist[b];
-    double f[27], ge[27];
-    pull_special(g, type, n, src, bst_cur + b, nb, f, ge);
-    tms_cell_sc(g, P, type, mom_cur, n, f, ge);
-#pragma unroll
-    for (int l = 0; l < 27; ++l) {
-        bst_nxt[(long)l * nb + b] = f[l];
-        bst_nxt[(long)(27 + l) * nb + b] = ge[l];
-    }
-    ScSums s;
-    sums_sc(f, ge, s);
+    if (cf != CF_FLUID) return;  // not fluid, or special (k_sc_special)
     store_record_sc(g, P, n, s, mom_nxt, status);
 }
 
@@ -351,10 +344,10 @@ int launch_collide(lbmgpu *h) {
     EvPair ep{};
     ev_begin(h, K_COLLIDE, ep);
     if (h->pack_mode != PK_STEPPED)
-        k_sc_collide<true><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(
+        k_sc_collide<true><<<grid_for(h->g.ncell), 2 * kBlock, 0, h->stream>>>(
             h->g, h->P, h->type, h->cflag, h->bid, h->pop[c], h->pop[x], h->mom[c], h->bst[c], h->nb, h->status);
     else
-        k_sc_collide<false><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(
+        k_sc_collide<false><<<grid_for(h->g.ncell), 2 * kBlock, 0, h->stream>>>(
             h->g, h->P, h->type, h->cflag, h->bid, h->pop[c], h->pop[x], h->mom[c], h->bst[c], h->nb, h->status);
     ev_end(h, ep);
     CK(cudaGetLastError());
@@ -364,20 +357,26 @@ int launch_collide(lbmgpu *h) {
 int launch_stream_moment(lbmgpu *h) {
     if (h->ns > 0) return lbmh::mc_launch_stream(h);
     const int c = h->cur, x = 1 - c;
+    // the special cells on the side stream beside the others: disjoint cells, both read only the
+    // collision's output and the previous record
+    if (h->nb > 0) {
+        CK(cudaEventRecord(h->fork, h->stream));
+        CK(cudaStreamWaitEvent(h->side, h->fork, 0));
+        EvPair eb{};
+        ev_begin(h, K_OTHER, eb, h->side);
+        k_sc_special<<<(unsigned)((h->nb + kScSpCells - 1) / kScSpCells), 2 * kScSpCells, 0, h->side>>>(
+            h->g, h->P, h->type, h->blist, h->pop[x], h->mom[c], h->mom[x], h->bst[c], h->bst[x], h->nb, h->status);
+        ev_end(h, eb, h->side);
+        CK(cudaGetLastError());
+        CK(cudaEventRecord(h->join, h->side));
+    }
     EvPair ep{};
     ev_begin(h, K_STREAM_MOMENT, ep);
     k_sc_stream_moment<<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(h->g, h->P, h->cflag, h->pop[x],
                                                                         h->mom[x], h->status);
     ev_end(h, ep);
     CK(cudaGetLastError());
-    if (h->nb > 0) {
-        EvPair eb{};
-        ev_begin(h, K_OTHER, eb);
-        k_sc_stream_moment_special<<<grid_for(h->nb), kBlock, 0, h->stream>>>(
-            h->g, h->P, h->type, h->blist, h->pop[x], h->mom[c], h->mom[x], h->bst[c], h->bst[x], h->nb, h->status);
-        ev_end(h, eb);
-        CK(cudaGetLastError());
-    }
+    if (h->nb > 0) CK(cudaStreamWaitEvent(h->stream, h->join, 0));
     h->cur = x;
     h->pack_mode = PK_STEPPED;
     return 0;

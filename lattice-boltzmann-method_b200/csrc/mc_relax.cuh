@@ -27,18 +27,6 @@
 
 namespace lbm {
 
-// direction of the axis indices (0, 1, 2 for c = 0, +1, -1)
-__host__ __device__ constexpr int dir3(int ix, int iy, int iz) {
-    constexpr int8_t t[27] = {0, 5, 6, 3, 11, 17, 4, 18, 12, 1, 9, 15, 7, 19, 21, 13, 23, 26, 2, 16, 10, 14, 25, 24, 8, 22, 20};
-    return t[9 * ix + 3 * iy + iz];
-}
-constexpr bool dir3_ok() {
-    for (int l = 0; l < 27; ++l)
-        if (dir3(cidx(cx(l)), cidx(cy(l)), cidx(cz(l))) != l) return false;
-    return true;
-}
-static_assert(dir3_ok(), "dir3 inverts cx, cy, cz");
-
 // Blocks of 128 threads per SM.  Five (96 registers) spill 340 B: 971 for 975 us in FP32, 111 for
 // 104 us in FP64.
 constexpr int kRelaxBlocks = 4;
