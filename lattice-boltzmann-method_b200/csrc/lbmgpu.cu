@@ -23,6 +23,7 @@
 #include "sc_special.cuh"
 #include "sums.cuh"
 #include "halo.cuh"
+#include "launch.cuh"
 
 using namespace lbm;
 using lbmh::MixOff;
@@ -65,9 +66,10 @@ __global__ void __launch_bounds__(2 * kBlock, 2)
     const int set = threadIdx.x / kBlock;  // 0: f, 1: g
     const long n = (long)blockIdx.x * kBlock + threadIdx.x % kBlock, nc = g.ncell;
     if (n >= nc) return;
-    const uint8_t cf = cflag[n];
     PullSrc ps;
     const long m = pull_interior(g, n, ps);
+    lbmh::step_begin();
+    const uint8_t cf = cflag[n];
     const double *const s0 = src + (long)27 * set * nc;
     double v[27];
 #pragma unroll
@@ -147,10 +149,11 @@ __global__ void __launch_bounds__(kBlock, 4)
                        double *__restrict__ mom_nxt, unsigned *status) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= g.ncell) return;
-    const uint8_t cf = cflag[n];
     const long nc = g.ncell;
     PullSrc ps;
     pull_interior(g, n, ps);
+    lbmh::step_begin();
+    const uint8_t cf = cflag[n];
     ScSums s;
     sums_init(s);
 #pragma unroll
@@ -343,12 +346,10 @@ int launch_collide(lbmgpu *h) {
     const int c = h->cur, x = 1 - c;
     EvPair ep{};
     ev_begin(h, K_COLLIDE, ep);
-    if (h->pack_mode != PK_STEPPED)
-        k_sc_collide<true><<<grid_for(h->g.ncell), 2 * kBlock, 0, h->stream>>>(
-            h->g, h->P, h->type, h->cflag, h->bid, h->pop[c], h->pop[x], h->mom[c], h->bst[c], h->nb, h->status);
-    else
-        k_sc_collide<false><<<grid_for(h->g.ncell), 2 * kBlock, 0, h->stream>>>(
-            h->g, h->P, h->type, h->cflag, h->bid, h->pop[c], h->pop[x], h->mom[c], h->bst[c], h->nb, h->status);
+    const bool stepped = h->pack_mode == PK_STEPPED;
+    CK(launch_next(!h->prof && h->nb == 0 && stepped, stepped ? k_sc_collide<false> : k_sc_collide<true>,
+                   grid_for(h->g.ncell), 2 * kBlock, 0, h->stream, h->g, h->P, h->type, h->cflag, h->bid, h->pop[c],
+                   h->pop[x], h->mom[c], h->bst[c], h->nb, h->status));
     ev_end(h, ep);
     CK(cudaGetLastError());
     return 0;
@@ -372,8 +373,8 @@ int launch_stream_moment(lbmgpu *h) {
     }
     EvPair ep{};
     ev_begin(h, K_STREAM_MOMENT, ep);
-    k_sc_stream_moment<<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(h->g, h->P, h->cflag, h->pop[x],
-                                                                        h->mom[x], h->status);
+    CK(launch_next(!h->prof && h->nb == 0, k_sc_stream_moment, grid_for(h->g.ncell), kBlock, 0, h->stream, h->g, h->P,
+                   h->cflag, h->pop[x], h->mom[x], h->status));
     ev_end(h, ep);
     CK(cudaGetLastError());
     if (h->nb > 0) CK(cudaStreamWaitEvent(h->stream, h->join, 0));

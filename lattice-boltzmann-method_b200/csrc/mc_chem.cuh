@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(kBlock, 2) k_mc_explicit(McArgsT<S, double> A)
 // has them for it (kinetics_h2_air_9.cuh): every cell (k_mc_chem) or the integrator list
 // (k_mc_chem_list).  Returns false when the handle's mechanism is not compiled.
 template <int NS>
-bool launch_compiled_chem(lbmgpu *h, const McArgs &A, unsigned grid, bool list) {
+bool launch_compiled_chem(lbmgpu *h, const McArgs &A, unsigned grid, bool list, cudaStream_t st) {
     if constexpr (NS == kin_h2_air_9::NS) {
         using KinH2 = kin_h2_air_9::Kinetics;
         if (h->kin != KIN_H2_AIR_9) return false;
@@ -113,17 +113,17 @@ bool launch_compiled_chem(lbmgpu *h, const McArgs &A, unsigned grid, bool list) 
             if (sm > 48 * 1024)
                 (void)cudaFuncSetAttribute(k_mc_chem_list<NS, KinH2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)sm);
-            k_mc_chem_list<NS, KinH2><<<grid, kBlock, sm, h->stream>>>(A);
+            k_mc_chem_list<NS, KinH2><<<grid, kBlock, sm, st>>>(A);
         } else if (A.sur.mode == 1) {
             if (sm > 48 * 1024)
                 (void)cudaFuncSetAttribute(k_mc_chem<NS, false, KinH2>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_mc_chem<NS, false, KinH2><<<grid, kBlock, sm, h->stream>>>(A);
+            k_mc_chem<NS, false, KinH2><<<grid, kBlock, sm, st>>>(A);
         } else {
             if (sm > 48 * 1024)
                 (void)cudaFuncSetAttribute(k_mc_chem<NS, false, KinH2, false>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            k_mc_chem<NS, false, KinH2, false><<<grid, kBlock, sm, h->stream>>>(A);
+            k_mc_chem<NS, false, KinH2, false><<<grid, kBlock, sm, st>>>(A);
         }
         return true;
     }
@@ -135,38 +135,41 @@ bool launch_compiled_chem(lbmgpu *h, const McArgs &A, unsigned grid, bool list) 
 namespace lbmh {
 
 template <int NS>
-int chem_step(lbmgpu *h, const lbm::McArgs &A) {
+int chem_step(lbmgpu *h, const lbm::McArgs &A, cudaStream_t st) {
     const unsigned gp = grid_for(h->g.ncell);
     EvPair ec{};
-    ev_begin(h, K_CHEM, ec);
+    ev_begin(h, K_CHEM, ec, st);
     if (A.sur.mode == 1 && A.sur.ilist)
-        k_mc_chem<NS, true><<<gp, kBlock, 0, h->stream>>>(A);
-    else if (!launch_compiled_chem<NS>(h, A, gp, false))
-        k_mc_chem<NS, false><<<gp, kBlock, 0, h->stream>>>(A);
-    ev_end(h, ec);
+        k_mc_chem<NS, true><<<gp, kBlock, 0, st>>>(A);
+    else if (!launch_compiled_chem<NS>(h, A, gp, false, st))
+        k_mc_chem<NS, false><<<gp, kBlock, 0, st>>>(A);
+    ev_end(h, ec, st);
     CK(cudaGetLastError());
     if (A.sur.ilist) {
         EvPair ei{};
-        ev_begin(h, K_SURROGATE, ei);
-        if (!launch_compiled_chem<NS>(h, A, 148 * 8, true))
-            k_mc_chem_list<NS><<<148 * 8, kBlock, 0, h->stream>>>(A);
-        ev_end(h, ei);
+        ev_begin(h, K_SURROGATE, ei, st);
+        if (!launch_compiled_chem<NS>(h, A, 148 * 8, true, st))
+            k_mc_chem_list<NS><<<148 * 8, kBlock, 0, st>>>(A);
+        ev_end(h, ei, st);
         CK(cudaGetLastError());
     }
     return 0;
 }
 
 template <int NS, typename S>
-int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A) {
+int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A, cudaStream_t st) {
     const unsigned gp = grid_for(h->g.ncell);
+    EvPair ec{};
+    ev_begin(h, K_PROPS, ec, st);
     bool compiled = false;
     if constexpr (NS == kin_h2_air_9::NS) {
         if (h->kin == KIN_H2_AIR_9) {
-            k_mc_explicit<NS, S, kin_h2_air_9::Kinetics><<<gp, kBlock, 0, h->stream>>>(A);
+            k_mc_explicit<NS, S, kin_h2_air_9::Kinetics><<<gp, kBlock, 0, st>>>(A);
             compiled = true;
         }
     }
-    if (!compiled) k_mc_explicit<NS, S, gas::DenseNet<NS>><<<gp, kBlock, 0, h->stream>>>(A);
+    if (!compiled) k_mc_explicit<NS, S, gas::DenseNet<NS>><<<gp, kBlock, 0, st>>>(A);
+    ev_end(h, ec, st);
     CK(cudaGetLastError());
     return 0;
 }

@@ -7,6 +7,7 @@
 // Measured: 96^3 FP32 storage 209 -> 144 us (152 us at four blocks per SM), 64 x 48 x 40 FP64
 // 55 -> 42 us (50 us at five blocks, which spill 120 B).
 #pragma once
+#include "launch.cuh"
 #include "mc_cell.cuh"
 
 namespace lbm {
@@ -16,6 +17,7 @@ __global__ void __launch_bounds__(128, sizeof(S) == sizeof(float) ? 5 : 4) k_mc_
     constexpr bool fast = sizeof(S) == sizeof(float);  // reciprocal densities and enthalpy quotients
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x, nc = A.ncell;
     if (n >= nc) return;
+    lbmh::step_begin();
     const unsigned cf = A.cflag[n];
     const long m = min(max(n, A.si), nc - 1 - A.si);  // n, if it is a fluid cell
     const gas::Tables &t = *A.tab;

@@ -21,6 +21,7 @@
 #include "handle.cuh"
 #include "mc_bc.cuh"
 #include "mc_cell.cuh"
+#include "launch.cuh"
 #include "mc_eflux.cuh"
 #include "mc_moments.cuh"
 #include "mc_ops.cuh"
@@ -41,6 +42,7 @@ using namespace lbmh;
 template <int NS, typename S>
 __global__ void __launch_bounds__(kBlock, 3) k_mc_props(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    lbmh::step_begin();
     if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
     mc_props_cell<NS, CHEM_OFF>(A, n);
 }
@@ -253,38 +255,43 @@ int collide_t(lbmgpu *h) {
     A.bst_cur = bstb<S>(h, c);
     const int rs_ = sur_prepare_t<S>(h, A);
     if (rs_) return rs_;
-    EvPair ep{};
-    ev_begin(h, K_PROPS, ep);
     const unsigned gp = grid_for(h->g.ncell);
-    k_mc_props<NS, S><<<gp, kBlock, 0, h->stream>>>(A);
-    if (h->chem == CHEM_REF_EXPLICIT) {
-        const int rc_ = explicit_step<NS, S>(h, A);
-        if (rc_) return rc_;
+    // The chemistry runs on the side stream beside the transport and energy-flux kernels: they read the
+    // same record and write different parameters, and on small lattices neither fills the device
+    // (8^3, explicit chemistry: 137 -> 97 us a step).  While kernels are timed they run in turn.
+    const bool beside = h->chem != CHEM_OFF && !h->prof;
+    if (beside) {
+        CK(cudaEventRecord(h->fork, h->stream));
+        CK(cudaStreamWaitEvent(h->side, h->fork, 0));
     }
-    ev_end(h, ep);
-    CK(cudaGetLastError());
-    if (h->chem == CHEM_ROSENBROCK) {
+    const cudaStream_t cs = beside ? h->side : h->stream;
+    if (h->chem == CHEM_REF_EXPLICIT) {
+        const int rc_ = explicit_step<NS, S>(h, A, cs);
+        if (rc_) return rc_;
+    } else if (h->chem == CHEM_ROSENBROCK) {
         McArgsT<double, double> C = base_args<double>(h);  // no populations in it: one instance for both storages
         C.rec_cur = A.rec_cur;
         C.rec_nxt = A.rec_nxt;
         C.sur = A.sur;
-        const int rc_ = chem_step<NS>(h, C);
+        const int rc_ = chem_step<NS>(h, C, cs);
         if (rc_) return rc_;
     }
+    if (beside) CK(cudaEventRecord(h->join, h->side));
+    EvPair ep{};
+    ev_begin(h, K_PROPS, ep);
+    // after the last step's moments, if nothing was put on the stream between
+    CK(launch_next(!h->prof && !beside && h->nb == 0 && !local, k_mc_props<NS, S>, gp, kBlock, 0, h->stream, A));
+    ev_end(h, ep);
     EvPair ee{};
     ev_begin(h, K_EFLUX, ee);
-    k_mc_eflux<NS, S><<<gp, kBlock, 0, h->stream>>>(A);
+    CK(launch_next(!h->prof, k_mc_eflux<NS, S>, gp, kBlock, 0, h->stream, A));
     ev_end(h, ee);
-    CK(cudaGetLastError());
+    if (beside) CK(cudaStreamWaitEvent(h->stream, h->join, 0));
     EvPair er{};
     ev_begin(h, K_COLLIDE, er);
-    const dim3 gr(grid_for(h->g.ncell), NS + 1);
-    if (h->chem == CHEM_OFF)
-        k_mc_relax<NS, false, S><<<gr, kBlock, 0, h->stream>>>(A);
-    else
-        k_mc_relax<NS, true, S><<<gr, kBlock, 0, h->stream>>>(A);
+    CK(launch_next(!h->prof && !beside, h->chem == CHEM_OFF ? k_mc_relax<NS, false, S> : k_mc_relax<NS, true, S>,
+                   dim3(gp, NS + 1), kBlock, 0, h->stream, A));
     ev_end(h, er);
-    CK(cudaGetLastError());
     return 0;
 }
 
@@ -311,15 +318,14 @@ int stream_t(lbmgpu *h) {
     }
     EvPair ep{};
     ev_begin(h, K_STREAM_MOMENT, ep);
-    k_mc_gather<NS, S><<<(unsigned)((h->g.ncell + kGatherCells - 1) / kGatherCells), kGatherCells *(NS + 1), 0, h->stream>>>(A);
+    CK(launch_next(!h->prof && h->nb == 0, k_mc_gather<NS, S>, (unsigned)((h->g.ncell + kGatherCells - 1) / kGatherCells),
+                   kGatherCells * (NS + 1), 0, h->stream, A));
     ev_end(h, ep);
-    CK(cudaGetLastError());
     EvPair es{};
     ev_begin(h, K_SOLVE, es);
-    k_mc_diffuse<NS, S><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(A);
-    k_mc_thermo<NS, S><<<grid_for(h->g.ncell), kBlock, 0, h->stream>>>(A);
+    CK(launch_next(!h->prof, k_mc_diffuse<NS, S>, grid_for(h->g.ncell), kBlock, 0, h->stream, A));
+    CK(launch_next(!h->prof, k_mc_thermo<NS, S>, grid_for(h->g.ncell), kBlock, 0, h->stream, A));
     ev_end(h, es);
-    CK(cudaGetLastError());
     if (h->nb > 0) CK(cudaStreamWaitEvent(h->stream, h->join, 0));
     return 0;
 }

@@ -16,6 +16,7 @@
 // 48 x 40 x 37 FP64: 45 -> 44 and 108 -> 73 us.  The diffusion kernel at two blocks per SM (198
 // registers): 367 for 344 us.
 #pragma once
+#include "launch.cuh"
 #include "mc_cell.cuh"
 
 namespace lbm {
@@ -51,6 +52,7 @@ __global__ void __launch_bounds__(kGatherCells *(NS + 1), sizeof(S) == sizeof(fl
     const int lane = threadIdx.x & 31, set = threadIdx.x >> 5;
     const long n = (long)blockIdx.x * kGatherCells + lane, nc = A.ncell;
     const bool in = n < nc;
+    lbmh::step_begin();
     const unsigned cf = in ? A.cflag[n] : 0u;
     unsigned X[3], Y[3], Z[3];
     interior_pull(A, in ? n : 0, X, Y, Z);
@@ -107,6 +109,7 @@ template <int NS, typename S>
 __global__ void __launch_bounds__(128, 3) k_mc_diffuse(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell) return;
+    lbmh::step_begin();
     const unsigned cf = A.cflag[n];
     // every load before the flag is known
     double *const R = A.rec_nxt;
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(128, 5) k_mc_thermo(McArgsT<S, double> A) {
     thermo_load(tab, t);
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell) return;
+    lbmh::step_begin();
     const unsigned cf = A.cflag[n];
     double *const R = A.rec_nxt;
     const double rho = rec(A, R, RM_RHO, n), rhoe = rec(A, R, RM_RHOE, n);

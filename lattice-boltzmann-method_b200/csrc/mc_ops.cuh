@@ -68,17 +68,18 @@ struct McOps {
     static int halo(lbmgpu *h, int face, int what, double *buf, bool pack);
     static constexpr int props_planes() { return lbm::pr_count<NS>(); }
 };
-// The chemistry of one collision, stiff and explicit (mc_chem.cuh, instantiated in mc_chem<NS>.cu).
+// The chemistry of one collision on stream st, stiff and explicit (mc_chem.cuh, instantiated in
+// mc_chem<NS>.cu).
 template <int NS>
-int chem_step(lbmgpu *h, const lbm::McArgs &A);
+int chem_step(lbmgpu *h, const lbm::McArgs &A, cudaStream_t st);
 template <int NS, typename S>
-int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A);
-extern template int explicit_step<9, double>(lbmgpu *, const lbm::McArgsT<double, double> &);
-extern template int explicit_step<9, float>(lbmgpu *, const lbm::McArgsT<float, double> &);
-extern template int explicit_step<6, double>(lbmgpu *, const lbm::McArgsT<double, double> &);
-extern template int explicit_step<6, float>(lbmgpu *, const lbm::McArgsT<float, double> &);
-extern template int chem_step<9>(lbmgpu *, const lbm::McArgs &);
-extern template int chem_step<6>(lbmgpu *, const lbm::McArgs &);
+int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A, cudaStream_t st);
+extern template int explicit_step<9, double>(lbmgpu *, const lbm::McArgsT<double, double> &, cudaStream_t);
+extern template int explicit_step<9, float>(lbmgpu *, const lbm::McArgsT<float, double> &, cudaStream_t);
+extern template int explicit_step<6, double>(lbmgpu *, const lbm::McArgsT<double, double> &, cudaStream_t);
+extern template int explicit_step<6, float>(lbmgpu *, const lbm::McArgsT<float, double> &, cudaStream_t);
+extern template int chem_step<9>(lbmgpu *, const lbm::McArgs &, cudaStream_t);
+extern template int chem_step<6>(lbmgpu *, const lbm::McArgs &, cudaStream_t);
 // The boundary cells of one streaming on the side stream (mc_special.cuh, instantiated in
 // mc_special<NS>.cu).
 template <int NS, typename S>

@@ -22,6 +22,7 @@
 // block) was slower: 1086 us for 975, FP64 178 us for 104 at 48 x 40 x 37 -- the copies of 4 and 8
 // bytes cost more issue slots than the latency they hide.
 #pragma once
+#include "launch.cuh"
 #include "mc_cell.cuh"
 #include "mc_moments.cuh"
 
@@ -220,6 +221,7 @@ template <int NS, bool CHEM, typename S>
 __global__ void __launch_bounds__(128, kRelaxBlocks) k_mc_relax(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int a = blockIdx.y;
+    lbmh::step_begin();
     __shared__ double sh[30];  // FP32 storage: the set's 27 shifts and their momentum
     if (sizeof(S) == sizeof(float) && threadIdx.x < 30)
         sh[threadIdx.x] = A.shift[threadIdx.x < 27 ? 27 * a + threadIdx.x : 27 * (NS + 1) + kGsPerSpecies * a + 1 + threadIdx.x - 27];
