@@ -29,16 +29,10 @@
 #pragma once
 #include "mc_bc.cuh"
 #include "mc_cell.cuh"
+#include "mc_moments.cuh"
 #include "mc_ops.cuh"
 
 namespace lbm {
-
-// direction with the components (x, y, z)
-__host__ __device__ constexpr int dir_of(int x, int y, int z) {
-    for (int l = 0; l < 27; ++l)
-        if (cx(l) == x && cy(l) == y && cz(l) == z) return l;
-    return 0;
-}
 
 constexpr int kSpCells = 32;  // cells of a block, one per lane
 // kinds of upstream cells, each a mask over the 27 directions
@@ -135,16 +129,9 @@ __device__ __forceinline__ int sp_T_from_u(SpBlock<NS> &B, const gas::Tables &t,
     return it_used;
 }
 
-// The thread's equilibrium in direction l from the factors of sp_target_axes: a species' feq_l
-// (its factors are G's P) or the energy set's geq_l.
-template <int NS>
-__device__ __forceinline__ double sp_eq(const SpBlock<NS> &B, int l, double rho, double rhoa, const AxisG<double> &G) {
-    if (B.set < NS) return rhoa * G.P[0][cidx(cx(l))] * G.P[1][cidx(cy(l))] * G.P[2][cidx(cz(l))];
-    return geq_l(l, rho, G);
-}
-
-// Per-axis factors of the thread's target set (mc_target_axes): a species' factors in G.P, or the
-// energy set's G.  Returns T in SI.
+// Per-axis factors of the thread's target set (mc_target_axes).  A species' equilibrium is the energy
+// set's with E = 1 and A = 0 (to the bit), so that both kinds of warp run the same code.  Returns T in
+// SI.
 template <int NS>
 __device__ __forceinline__ double sp_target_axes(SpBlock<NS> &B, const gas::Tables &t, const UnitsF &U, double rho,
                                                  double rhoa, const double vel[3], const double vela[3], double T_lat,
@@ -163,7 +150,9 @@ __device__ __forceinline__ double sp_target_axes(SpBlock<NS> &B, const gas::Tabl
             G.P[d][0] = 1.0 - z;
             G.P[d][1] = (vela[d] + z) * 0.5;
             G.P[d][2] = (-vela[d] + z) * 0.5;
+            G.A[d][0] = G.A[d][1] = G.A[d][2] = 0.0;
         }
+        G.E = 1.0;
     } else {
         const double e = u_energy_mass(U, (float)(B.sum_w(0, t) * gas::kR * T_si));
         const double theta = u_energy_mass(U, (float)(gas::kR * T_si / W));
@@ -237,7 +226,7 @@ __device__ __forceinline__ void sp_nscbc_outflow(SpBlock<NS> &B, const AT &A, bo
         } else {
             if (!(Nax[d] - 2 > 3)) continue;
             any_t = true;
-            const int lo = d == 0 ? dir_of(1, 0, 0) : (d == 1 ? dir_of(0, 1, 0) : dir_of(0, 0, 1));
+            const int lo = d == 0 ? dir3(1, 0, 0) : (d == 1 ? dir3(0, 1, 0) : dir3(0, 0, 1));
             if (!((fluid_up >> lo) & 1))
                 mode = 1;
             else if (d != 2 && !((fluid_up >> opp(lo)) & 1))
@@ -538,7 +527,7 @@ __device__ __forceinline__ void sp_moments(SpBlock<NS> &B, const AT &A, long n, 
     const double vol = 1.0 / (double)si_rho(A.U, (float)rho);
     const double rho_n_si = 1.0 / vol;
     double Tn;
-    const int it = sp_T_from_u<NS, fast>(B, t, Y, u_si, T_si, 1e-14, 100, true, Tn);
+    const int it = sp_T_from_u<NS, fast>(B, t, Y, u_si, T_si, kNewtonTol, 100, true, Tn);
     const double Pn = rho_n_si * gas::kR * Tn / Wn;
     const double Tl = u_temp(A.U, (float)Tn);
     if (!valid) return;
@@ -639,14 +628,14 @@ __global__ void __launch_bounds__(kSpCells *(NS + 1), 1)
             for (int l = 1; l < 27; ++l) {
                 if (!((slip_m >> l) & 1)) continue;
                 int in = i - cx(l), jn = j - cy(l), kn = k - cz(l), lp = l;
-                if (cx(l) && ((slip_m >> dir_of(cx(l), 0, 0)) & 1)) {
-                    lp = dir_of(-cx(l), cy(l), cz(l));
+                if (cx(l) && ((slip_m >> dir3(cidx(cx(l)), 0, 0)) & 1)) {
+                    lp = dir3(cidx(-cx(l)), cidx(cy(l)), cidx(cz(l)));
                     in = i;
-                } else if (cy(l) && ((slip_m >> dir_of(0, cy(l), 0)) & 1)) {
-                    lp = dir_of(cx(l), -cy(l), cz(l));
+                } else if (cy(l) && ((slip_m >> dir3(0, cidx(cy(l)), 0)) & 1)) {
+                    lp = dir3(cidx(cx(l)), cidx(-cy(l)), cidx(cz(l)));
                     jn = j;
-                } else if (cz(l) && ((slip_m >> dir_of(0, 0, cz(l))) & 1)) {
-                    lp = dir_of(cx(l), cy(l), -cz(l));
+                } else if (cz(l) && ((slip_m >> dir3(0, 0, cidx(cz(l)))) & 1)) {
+                    lp = dir3(cidx(cx(l)), cidx(cy(l)), cidx(-cz(l)));
                     kn = k;
                 }
                 if (!((in == 0 && A.halo_lo) || (in == A.Nx - 1 && A.halo_hi)))
@@ -729,9 +718,22 @@ __global__ void __launch_bounds__(kSpCells *(NS + 1), 1)
             AxisG<double> G;
             const double Tsi = sp_target_axes(B, t, A.U, rho_x, rhoa_x, vel_x, vela_x, T_x, G);
             double m[3] = {0.0, 0.0, 0.0}, s0 = 0.0;
+            // e_l = B p_z + C A_z, B and C of the pair (c_x, c_y); the sums below in the reference's order
+            const double r = set < NS ? rhoa_x : rho_x;
+            double Bp[3][3], Cp[3][3];
+#pragma unroll
+            for (int ix = 0; ix < 3; ++ix) {
+                const double px = r * G.P[0][ix], tx = r * (G.E * G.P[0][ix] + G.A[0][ix]);
+#pragma unroll
+                for (int iy = 0; iy < 3; ++iy) {
+                    Bp[ix][iy] = tx * G.P[1][iy] + px * G.A[1][iy];
+                    Cp[ix][iy] = px * G.P[1][iy];
+                }
+            }
 #pragma unroll
             for (int l = 0; l < 27; ++l) {
-                const double e = sp_eq(B, l, rho_x, rhoa_x, G);
+                const int ix = cidx(cx(l)), iy = cidx(cy(l)), iz = cidx(cz(l));
+                const double e = Bp[ix][iy] * G.P[2][iz] + Cp[ix][iy] * G.A[2][iz];
                 const bool bd = (bm >> l) & 1;
                 if (stage == 0) {
                     const double fv = bd ? e : f[l];
