@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "handle.cuh"
+#include "launch.cuh"
 #include "mc_cell.cuh"
 #include "surrogate_host.cuh"
 
@@ -160,6 +161,13 @@ __global__ void k_sur_standardise(const float *__restrict__ x, long m, long mpad
     }
     X[r * kSurInX + kSurBiasSlot] = __float2bfloat16(1.0f);
     X[r * kSurInX + kSurInPad + kSurBiasSlot] = __float2bfloat16(1.0f);
+}
+
+// The kSurOut real outputs of n prediction rows, packed.
+__global__ void k_sur_pack(const float *__restrict__ pred, long n, float *__restrict__ out) {
+    static_assert(kSurOut <= kSurIn, "the packed outputs take the inputs' place");
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n * kSurOut) out[i] = pred[i / kSurOut * kSurOutPad + i % kSurOut];
 }
 
 struct SurNet {  // device pointers of the BF16 weights and FP32 biases
@@ -472,6 +480,7 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const __nv_bfloat16 *__restrict
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t *>(sm + kGmSlot);
+    step_begin();
     uint32_t phase[2] = {0u, 0u};
     bool pending[2] = {false, false};  // a commit of the stage not yet waited for
     bool ok = true;
@@ -538,15 +547,17 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const __nv_bfloat16 *__restrict
             uint32_t v[16];
             tc_ld16(trow + (uint32_t)(cb * 16), v);
             tc_wait_ld();
-            if (r < M)
+            // 16 columns are all inside or all outside (N a multiple of 16), rows 16-byte aligned (ldc
+            // and zstride multiples of 4): four words a store
+            if (r < M && n0 + cb * 16 < N) {
+                float4 *dst = reinterpret_cast<float4 *>(C + r * ldc + n0 + cb * 16);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int c = n0 + cb * 16 + j;
-                    if (c < N) {
-                        float *dst = C + r * ldc + c;
-                        *dst = __uint_as_float(v[j]) + (accum ? *dst : 0.f);
-                    }
+                for (int j = 0; j < 4; ++j) {
+                    const float4 o = accum ? dst[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    dst[j] = make_float4(__uint_as_float(v[4 * j]) + o.x, __uint_as_float(v[4 * j + 1]) + o.y,
+                                         __uint_as_float(v[4 * j + 2]) + o.z, __uint_as_float(v[4 * j + 3]) + o.w);
                 }
+            }
         }
     }
     if (!ok && tid == 0) atomicOr(status, (unsigned)LBMGPU_ST_SURROGATE);
@@ -561,6 +572,7 @@ __global__ void __launch_bounds__(128) k_gemm_tn(const __nv_bfloat16 *__restrict
 __global__ void k_sum_splits(const float *__restrict__ part, int splits, long n, int cols, int ld,
                              float *__restrict__ out) {
     const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    step_begin();
     if (e >= n || (int)(e % ld) >= cols) return;
     float v = 0.f;
     for (int z = 0; z < splits; ++z) v += part[(long)z * n + e];
@@ -571,6 +583,7 @@ __global__ void k_sum_splits(const float *__restrict__ part, int splits, long n,
 __global__ void k_bias_gelu(const float *__restrict__ C, const float *__restrict__ b, float *__restrict__ Z,
                             __nv_bfloat16 *__restrict__ H, long rows, int W) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    step_begin();
     if (i >= rows * W) return;
     const float z = C[i] + b[i % W];
     Z[i] = z;
@@ -578,12 +591,13 @@ __global__ void k_bias_gelu(const float *__restrict__ C, const float *__restrict
 }
 
 // Output layer: out = C + b4; dOut = 2 (out - y) / (valid * kSurOut) on the valid rows and
-// real outputs, 0 elsewhere; the squared errors summed per block into part[].
+// real outputs, 0 elsewhere, and its BF16 copy; the squared errors summed per block into part[].
 __global__ void k_out_loss(const float *__restrict__ C, const float *__restrict__ b4, const float *__restrict__ Yt,
                            const uint8_t *__restrict__ valid, float nvalid, float *__restrict__ dOut,
-                           double *__restrict__ part, long rows) {
+                           __nv_bfloat16 *__restrict__ dOutb, double *__restrict__ part, long rows) {
     __shared__ double red[256];
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    step_begin();
     double se = 0.0;
     if (i < rows * kSurOutPad) {
         const long r = i / kSurOutPad;
@@ -595,6 +609,7 @@ __global__ void k_out_loss(const float *__restrict__ C, const float *__restrict_
             g = 2.f * e / (nvalid * kSurOut);
         }
         dOut[i] = g;
+        dOutb[i] = __float2bfloat16(g);
     }
     red[threadIdx.x] = se;
     __syncthreads();
@@ -609,6 +624,7 @@ __global__ void k_out_loss(const float *__restrict__ C, const float *__restrict_
 __global__ void k_gelu_bwd(const float *__restrict__ dH, const float *__restrict__ Z, float *__restrict__ dZ,
                            __nv_bfloat16 *__restrict__ dZb, long n) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    step_begin();
     if (i >= n) return;
     const float g = dH[i] * gelu_grad(Z[i]);
     dZ[i] = g;
@@ -625,6 +641,7 @@ __global__ void k_transpose_bf16(const __nv_bfloat16 *__restrict__ in, int ldi, 
                                  int ldo, int rows, int cols) {
     __shared__ __nv_bfloat16 tile[32][33];
     const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
+    step_begin();
     for (int y = threadIdx.y; y < 32; y += blockDim.y) {
         const int r = by + y, c = bx + threadIdx.x;
         tile[y][threadIdx.x] = (r < rows && c < cols) ? in[(long)r * ldi + c] : __float2bfloat16(0.f);
@@ -636,31 +653,58 @@ __global__ void k_transpose_bf16(const __nv_bfloat16 *__restrict__ in, int ldi, 
     }
 }
 
-// db[c] = sum_r dZ[r][c] for a block of 32 columns: lane = column, warp w sums rows
-// w, w + 8, ... in order (a warp reads 32 consecutive floats of a row), then the 8 warp
-// sums are added in warp order -- a fixed order, so the result does not vary run to run.
-constexpr int kColsumWarps = 8;
-__global__ void __launch_bounds__(32 * kColsumWarps) k_colsum(const float *__restrict__ dZ, long rows, int W,
-                                                               float *__restrict__ db) {
-    __shared__ double part[kColsumWarps][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+// db[c] = sum_r dZ[r][c], in a fixed order, so that the result does not vary run to run: slice w of
+// eight (blockIdx.y) adds the rows w, w + 8, ... in FP64, then the slices are added in their order by the
+// last of a column group's (blockIdx.x, 32 columns) blocks to finish.  A block's 256 threads stage 256
+// rows at a time into shared memory for the one warp that adds them: the additions are a chain, and
+// with one thread per chain also loading, the kernel was a chain of memory latencies (75 us, four times
+// a batch of 480 us).
+constexpr int kColsumSlices = 8, kColsumRows = 256;
+__global__ void __launch_bounds__(256) k_colsum(const float *__restrict__ dZ, long rows, int W, double *__restrict__ part,
+                                                unsigned *__restrict__ done, float *__restrict__ db) {
+    __shared__ float tile[kColsumRows][32];
+    __shared__ unsigned ticket;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane, w = blockIdx.y;
+    step_begin();
     double s = 0.0;
-    if (c < W)
-        for (long r = warp; r < rows; r += kColsumWarps) s += dZ[r * W + c];
-    part[warp][lane] = s;
-    __syncthreads();
-    if (warp == 0 && c < W) {
+    for (long r0 = w; r0 < rows; r0 += (long)kColsumRows * kColsumSlices) {
+#pragma unroll 16
+        for (int q = warp; q < kColsumRows; q += 8) {
+            const long r = r0 + (long)q * kColsumSlices;
+            tile[q][lane] = r < rows && c < W ? dZ[r * W + c] : 0.f;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            const long left = (rows - r0 + kColsumSlices - 1) / kColsumSlices;
+            const int n = left < kColsumRows ? (int)left : kColsumRows;
+#pragma unroll 8
+            for (int q = 0; q < n; ++q) s += tile[q][lane];
+        }
+        __syncthreads();
+    }
+    if (warp != 0) return;
+    if (c < W) part[w * W + c] = s;
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) ticket = atomicAdd(&done[blockIdx.x], 1u);
+    __syncwarp();
+    if (ticket != kColsumSlices - 1) return;
+    __threadfence();
+    if (c < W) {
         double t = 0.0;
-        for (int w = 0; w < kColsumWarps; ++w) t += part[w][lane];
+        for (int q = 0; q < kColsumSlices; ++q) t += __ldcg(part + q * W + c);
         db[c] = (float)t;
     }
+    if (lane == 0) done[blockIdx.x] = 0u;  // for the next launch
 }
 
-// Adam on FP32 master parameters; the BF16 copy (if any) follows.  g at gradient stride.
+// Adam on the FP32 master parameters, all tensors in one launch; the BF16 copy of the weights (the
+// first nw elements) follows.
 __global__ void k_adam(float *__restrict__ w, float *__restrict__ m, float *__restrict__ v,
-                       const float *__restrict__ g, __nv_bfloat16 *__restrict__ wb, long n, float lr, float b1,
+                       const float *__restrict__ g, __nv_bfloat16 *__restrict__ wb, long n, long nw, float lr, float b1,
                        float b2, float c1, float c2, float eps) {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    step_begin();
     if (i >= n) return;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.f - b1) * gi;
@@ -669,24 +713,24 @@ __global__ void k_adam(float *__restrict__ w, float *__restrict__ m, float *__re
     v[i] = vi;
     const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     w[i] = wi;
-    if (wb) wb[i] = __float2bfloat16(wi);
+    if (i < nw) wb[i] = __float2bfloat16(wi);
 }
 
 // Batch rows from the sample set: network input rows and standardised FP32 targets.
 __global__ void k_gather_batch(const float *__restrict__ dx, const float *__restrict__ dy, const int *__restrict__ idx,
                                int nb, int B, const SurNorm *__restrict__ nrm, __nv_bfloat16 *__restrict__ Xb,
                                float *__restrict__ Yb, uint8_t *__restrict__ vb) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    // one thread per (row, slot): 16 neighbouring threads write a row's 16 slots
+    static_assert(kSurInPad == 16 && kSurOutPad == 16, "16 slots of input and output");
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, r = t >> 4, q = t & 15;
+    step_begin();
     if (r >= B) return;
     const bool ok = r < nb;
     const long s = ok ? idx[r] : 0;
-    for (int q = 0; q < kSurInPad; ++q) {
-        const float v = (ok && q < kSurIn) ? (dx[s * kSurIn + q] - nrm->x_mean[q]) / nrm->x_std[q] : 0.f;
-        put_split(Xb + (long)r * kSurInX, q, v);
-    }
-    for (int q = 0; q < kSurOutPad; ++q)
-        Yb[(long)r * kSurOutPad + q] = (ok && q < kSurOut) ? (dy[s * kSurOut + q] - nrm->y_mean[q]) / nrm->y_std[q] : 0.f;
-    vb[r] = ok ? 1 : 0;
+    const float v = (ok && q < kSurIn) ? (dx[s * kSurIn + q] - nrm->x_mean[q]) / nrm->x_std[q] : 0.f;
+    put_split(Xb + (long)r * kSurInX, q, v);
+    Yb[(long)r * kSurOutPad + q] = (ok && q < kSurOut) ? (dy[s * kSurOut + q] - nrm->y_mean[q]) / nrm->y_std[q] : 0.f;
+    if (q == 0) vb[r] = ok ? 1 : 0;
 }
 
 // State-space augmentation.  New row i takes a random valid row of the sample set (the
@@ -742,11 +786,10 @@ __global__ void k_sur_augment(const gas::Tables *__restrict__ tab, float *__rest
 inline unsigned blocks(long n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
 // k_gemm_tn over the whole C (splits > 1: split K, partials zstride apart).
-void gemm_tn(lbmgpu *h, const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *Bm, int ldb, float *C, int ldc, int M,
-             int N, int K, int accum = 0, int splits = 1, long zstride = 0) {
-    cudaFuncSetAttribute(k_gemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmSmem);
-    k_gemm_tn<<<dim3((N + kGmN - 1) / kGmN, (M + kGmM - 1) / kGmM, splits), 128, kGmSmem, h->stream>>>(
-        A, lda, Bm, ldb, C, ldc, M, N, K, accum, zstride, h->status);
+cudaError_t gemm_tn(lbmgpu *h, const __nv_bfloat16 *A, int lda, const __nv_bfloat16 *Bm, int ldb, float *C, int ldc, int M,
+                    int N, int K, int accum = 0, int splits = 1, long zstride = 0) {
+    return launch_next(true, k_gemm_tn, dim3((N + kGmN - 1) / kGmN, (M + kGmM - 1) / kGmM, splits), 128, kGmSmem, h->stream,
+                       A, lda, Bm, ldb, C, ldc, M, N, K, accum, zstride, h->status);
 }
 
 }  // namespace
@@ -781,6 +824,20 @@ struct SurState {
     bool trained = false;
     long adam_t = 0, train_steps = 0;
     double last_loss = 0.0;
+    // training buffers, kept between calls of the same batch size (freed with the handle): 4 kB per
+    // batch row and 4 B per sample row
+    struct Work {
+        int B = 0;
+        long rows = 0, nbatch = 0;
+        int *idx = nullptr;
+        __nv_bfloat16 *Xb = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *dZb = nullptr, *T1 = nullptr,
+                      *T2 = nullptr, *Wt = nullptr;
+        float *Yb = nullptr, *C = nullptr, *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *dA = nullptr, *Gp = nullptr;
+        uint8_t *vb = nullptr;
+        double *part = nullptr, *csum = nullptr;  // loss partials; bias gradients: slice sums, blocks done
+        unsigned *cdone = nullptr;
+        size_t bytes = 0;
+    } work;
 };
 
 namespace {
@@ -889,9 +946,20 @@ int sur_create(lbmgpu *h) {
     return init_params(h, 20261203u);
 }
 
+static void work_release(lbmgpu *h, SurState &s) {
+    SurState::Work &w = s.work;
+    for (void *p : {(void *)w.idx, (void *)w.Xb, (void *)w.H1, (void *)w.H2, (void *)w.H3, (void *)w.dZb, (void *)w.T1,
+                    (void *)w.T2, (void *)w.Wt, (void *)w.Yb, (void *)w.C, (void *)w.Z1, (void *)w.Z2, (void *)w.Z3,
+                    (void *)w.dA, (void *)w.Gp, (void *)w.vb, (void *)w.part, (void *)w.csum, (void *)w.cdone})
+        cudaFree(p);
+    h->bytes -= w.bytes;
+    w = SurState::Work{};
+}
+
 void sur_release(lbmgpu *h) {
     SurState *s = h->sur;
     if (!s) return;
+    work_release(h, *s);
     cudaFree(s->w);
     cudaFree(s->m);
     cudaFree(s->v);
@@ -1208,13 +1276,6 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
         if (v[r]) rows.push_back((int)r);
     if (rows.size() < 2) return LBMGPU_E_STATE;
     const int B = batch;
-    // batch buffers
-    int *idx = nullptr;
-    __nv_bfloat16 *Xb = nullptr, *H1 = nullptr, *H2 = nullptr, *H3 = nullptr, *dZb = nullptr, *T1 = nullptr,
-                  *T2 = nullptr, *Wt = nullptr;
-    float *Yb = nullptr, *C = nullptr, *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *dA = nullptr, *dZ = nullptr;
-    uint8_t *vb = nullptr;
-    double *part = nullptr;
     const long BH = (long)B * kSurHid;
     const unsigned nparts = blocks((long)B * kSurOutPad);
     const long nbatch = ((long)rows.size() + B - 1) / B, total = std::max<long>(1, (long)epochs * nbatch);
@@ -1224,31 +1285,71 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
             ksplit = c;
             break;
         }
-    float *Gp = nullptr;  // the weight gradients' split-K partials
-    auto all = [&]() {
-        int r = dalloc(h, &idx, rows.size());
-        if (!r) r = dalloc(h, &Xb, (size_t)B * kSurInX);
-        if (!r) r = dalloc(h, &Yb, (size_t)B * kSurOutPad);
-        if (!r) r = dalloc(h, &vb, B);
-        if (!r) r = dalloc(h, &H1, BH);
-        if (!r) r = dalloc(h, &H2, BH);
-        if (!r) r = dalloc(h, &H3, BH);
-        if (!r) r = dalloc(h, &Z1, BH);
-        if (!r) r = dalloc(h, &Z2, BH);
-        if (!r) r = dalloc(h, &Z3, BH);
-        if (!r) r = dalloc(h, &C, BH);
-        if (!r) r = dalloc(h, &dA, BH);
-        if (!r) r = dalloc(h, &dZ, BH);
-        if (!r) r = dalloc(h, &dZb, BH);
-        if (!r) r = dalloc(h, &T1, BH);
-        if (!r) r = dalloc(h, &T2, BH);
-        if (!r) r = dalloc(h, &Wt, (size_t)kSurHid * kSurLd);
-        if (!r) r = dalloc(h, &part, (size_t)nparts * nbatch);
-        if (!r) r = dalloc(h, &Gp, (size_t)ksplit * kSurHid * kSurLd);
-        if (!r && cudaMemsetAsync(Gp, 0, (size_t)ksplit * kSurHid * kSurLd * sizeof(float), h->stream)) r = LBMGPU_E_CUDA;
-        return r;
+    SurState::Work &wk = s.work;
+    const size_t gp_n = (size_t)ksplit * kSurHid * kSurLd;  // the weight gradients' split-K partials
+    if (wk.B != B || wk.rows < (long)rows.size() || wk.nbatch < nbatch) {
+        work_release(h, s);
+        const size_t before = h->bytes;
+        int r = dalloc(h, &wk.idx, rows.size());
+        if (!r) r = dalloc(h, &wk.Xb, (size_t)B * kSurInX);
+        if (!r) r = dalloc(h, &wk.Yb, (size_t)B * kSurOutPad);
+        if (!r) r = dalloc(h, &wk.vb, B);
+        if (!r) r = dalloc(h, &wk.H1, BH);
+        if (!r) r = dalloc(h, &wk.H2, BH);
+        if (!r) r = dalloc(h, &wk.H3, BH);
+        if (!r) r = dalloc(h, &wk.Z1, BH);
+        if (!r) r = dalloc(h, &wk.Z2, BH);
+        if (!r) r = dalloc(h, &wk.Z3, BH);
+        if (!r) r = dalloc(h, &wk.C, BH);
+        if (!r) r = dalloc(h, &wk.dA, BH);
+        if (!r) r = dalloc(h, &wk.dZb, BH);
+        if (!r) r = dalloc(h, &wk.T1, BH);
+        if (!r) r = dalloc(h, &wk.T2, BH);
+        if (!r) r = dalloc(h, &wk.Wt, (size_t)kSurHid * kSurLd);
+        if (!r) r = dalloc(h, &wk.part, (size_t)nparts * nbatch);
+        if (!r) r = dalloc(h, &wk.Gp, gp_n);
+        if (!r) r = dalloc(h, &wk.csum, (size_t)kColsumSlices * kSurHid);
+        if (!r) r = dalloc(h, &wk.cdone, kSurHid / 32);
+        if (!r && cudaMemsetAsync(wk.cdone, 0, kSurHid / 32 * sizeof(unsigned), h->stream)) r = LBMGPU_E_CUDA;
+        wk.bytes = h->bytes - before;
+        if (r) {
+            work_release(h, s);
+            return r;
+        }
+        wk.B = B;
+        wk.rows = (long)rows.size();
+        wk.nbatch = nbatch;
+    }
+    int *const idx = wk.idx;
+    __nv_bfloat16 *const Xb = wk.Xb, *const H1 = wk.H1, *const H2 = wk.H2, *const H3 = wk.H3, *const dZb = wk.dZb,
+                  *const T1 = wk.T1, *const T2 = wk.T2, *const Wt = wk.Wt;
+    float *const Yb = wk.Yb, *const C = wk.C, *const Z1 = wk.Z1, *const Z2 = wk.Z2, *const Z3 = wk.Z3, *const dA = wk.dA,
+          *const Gp = wk.Gp;
+    uint8_t *const vb = wk.vb;
+    double *const part = wk.part;
+    CK(cudaFuncSetAttribute(k_gemm_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGmSmem));
+    CK(cudaMemsetAsync(Gp, 0, gp_n * sizeof(float), h->stream));
+    rc = 0;
+    // a batch's kernels, each launched while the one before drains (launch.cuh); the first refusal is kept
+    auto run = [&](auto kernel, dim3 grid, dim3 block, auto... args) {
+        if (rc) return;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = grid;
+        cfg.blockDim = block;
+        cfg.stream = h->stream;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+        if (e != cudaSuccess) rc = cuda_fail(e);
     };
-    rc = all();
+    auto gemm = [&](auto... args) {
+        if (rc) return;
+        const cudaError_t e = gemm_tn(h, args...);
+        if (e != cudaSuccess) rc = cuda_fail(e);
+    };
     std::mt19937_64 rng(seed);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     SurNet net = net_of(s);
@@ -1272,7 +1373,8 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
         long bi = 0;
         for (size_t b0 = 0; b0 < rows.size() && !rc; b0 += B, ++bi) {
             const int nb = (int)std::min<size_t>(B, rows.size() - b0);
-            k_gather_batch<<<blocks(B), 256, 0, h->stream>>>(s.ds_x, s.ds_y, idx + b0, nb, B, s.nrm, Xb, Yb, vb);
+            run(k_gather_batch, blocks((long)B * 16), 256, (const float *)s.ds_x, (const float *)s.ds_y,
+                (const int *)(idx + b0), nb, B, (const SurNorm *)s.nrm, Xb, Yb, vb);
             // forward
             const __nv_bfloat16 *in = Xb;
             __nv_bfloat16 *Hs[3] = {H1, H2, H3};
@@ -1280,37 +1382,37 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
             const __nv_bfloat16 *Ws[4] = {net.w1, net.w2, net.w3, net.w4};
             const float *bs[4] = {net.b1, net.b2, net.b3, net.b4};
             for (int L = 0; L < 3; ++L) {
-                gemm_tn(h, in, L == 0 ? kSurInX : kSurHid, Ws[L], ldw[L], C, kSurHid, B, nout[L], kin[L]);
+                gemm(in, L == 0 ? kSurInX : kSurHid, Ws[L], ldw[L], C, kSurHid, B, nout[L], kin[L]);
                 if (L == 0)  // the remainders' share of the first layer
-                    gemm_tn(h, Xb + kSurInPad, kSurInX, Ws[0], ldw[0], C, kSurHid, B, nout[0], kin[0], 1);
-                k_bias_gelu<<<blocks(BH), 256, 0, h->stream>>>(C, bs[L], Zs[L], Hs[L], B, kSurHid);
+                    gemm(Xb + kSurInPad, kSurInX, Ws[0], ldw[0], C, kSurHid, B, nout[0], kin[0], 1);
+                run(k_bias_gelu, blocks(BH), 256, (const float *)C, bs[L], Zs[L], Hs[L], (long)B, kSurHid);
                 in = Hs[L];
             }
-            gemm_tn(h, H3, kSurHid, net.w4, kSurLd, C, kSurOutPad, B, kSurOutPad, kSurHid);
-            k_out_loss<<<nparts, 256, 0, h->stream>>>(C, net.b4, Yb, vb, (float)nb, dA, part + (size_t)bi * nparts, B);
-            // backward: dA holds dL/d(pre-activation) of the current layer (FP32), rows x nout
+            gemm(H3, kSurHid, net.w4, kSurLd, C, kSurOutPad, B, kSurOutPad, kSurHid);
+            run(k_out_loss, nparts, 256, (const float *)C, net.b4, (const float *)Yb, (const uint8_t *)vb, (float)nb, dA, dZb,
+                part + (size_t)bi * nparts, (long)B);
+            // backward: dA holds dL/d(pre-activation) of the current layer (FP32), rows x nout, dZb its
+            // BF16 copy
             float *gw[4] = {s.g + off_w(0), s.g + off_w(1), s.g + off_w(2), s.g + off_w(3)};
             float *gb[4] = {s.g + off_w(4), s.g + off_w(5), s.g + off_w(6), s.g + off_w(7)};
             for (int L = 3; L >= 0; --L) {
                 const int no = nout[L], ki = kin[L];
                 // bias gradient
-                k_colsum<<<(no + 31) / 32, 32 * kColsumWarps, 0, h->stream>>>(dA, B, no, gb[L]);
+                run(k_colsum, dim3((no + 31) / 32, kColsumSlices), 256, (const float *)dA, (long)B, no, wk.csum, wk.cdone, gb[L]);
                 // dZ^T [no][B] and input^T [ki][B] for the weight gradient dW = dZ^T in
-                k_f32_to_bf16<<<blocks((long)B * no), 256, 0, h->stream>>>(dA, dZb, (long)B * no);
-                k_transpose_bf16<<<dim3((no + 31) / 32, (B + 31) / 32), tb, 0, h->stream>>>(dZb, no, T1, B, B, no);
+                run(k_transpose_bf16, dim3((no + 31) / 32, (B + 31) / 32), tb, (const __nv_bfloat16 *)dZb, no, T1, B, B, no);
                 const __nv_bfloat16 *inp = L == 0 ? Xb : Hs[L - 1];
-                k_transpose_bf16<<<dim3((ki + 31) / 32, (B + 31) / 32), tb, 0, h->stream>>>(
-                    inp, L == 0 ? kSurInX : kSurHid, T2, B, B, ki);  // layer 0: the values' columns
+                run(k_transpose_bf16, dim3((ki + 31) / 32, (B + 31) / 32), tb, inp, L == 0 ? kSurInX : kSurHid, T2, B, B,
+                    ki);  // layer 0: the values' columns
                 // split K (the batch) so the small weight-gradient tile keeps every SM busy
                 const long gsz = (long)no * ldw[L];
-                gemm_tn(h, T1, B, T2, B, Gp, ldw[L], no, ki, B, 0, ksplit, gsz);
-                k_sum_splits<<<blocks(gsz), 256, 0, h->stream>>>(Gp, ksplit, gsz, ki, ldw[L], gw[L]);
+                gemm(T1, B, T2, B, Gp, ldw[L], no, ki, B, 0, ksplit, gsz);
+                run(k_sum_splits, blocks(gsz), 256, (const float *)Gp, ksplit, gsz, ki, ldw[L], gw[L]);
                 if (L == 0) break;
                 // dH_prev = dZ W  (W^T [ki][no] as the B operand), then through GELU'
-                k_transpose_bf16<<<dim3((ki + 31) / 32, (no + 31) / 32), tb, 0, h->stream>>>(Ws[L], ldw[L], Wt, kSurLd,
-                                                                                              no, ki);
-                gemm_tn(h, dZb, no, Wt, kSurLd, C, kSurHid, B, ki, no);
-                k_gelu_bwd<<<blocks(BH), 256, 0, h->stream>>>(C, Zs[L - 1], dA, T1, BH);
+                run(k_transpose_bf16, dim3((ki + 31) / 32, (no + 31) / 32), tb, Ws[L], ldw[L], Wt, kSurLd, no, ki);
+                gemm(dZb, no, Wt, kSurLd, C, kSurHid, B, ki, no);
+                run(k_gelu_bwd, blocks(BH), 256, (const float *)C, (const float *)Zs[L - 1], dA, dZb, BH);
             }
             // Adam step over every parameter (padding entries have zero gradient)
             s.adam_t += 1;
@@ -1318,17 +1420,9 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
                 (float)(0.5 * lr * (1.0 + std::cos(3.14159265358979323846 * (double)step_in_call / (double)total)));
             ++step_in_call;
             const float c1 = 1.f - (float)std::pow(b1, (double)s.adam_t), c2 = 1.f - (float)std::pow(b2, (double)s.adam_t);
-            for (int t = 0; t < 8; ++t) {
-                const size_t sz[8] = {kW1, kW2, kW2, kW4, kSurHid, kSurHid, kSurHid, kSurOutPad};
-                const size_t o = off_w(t);
-                k_adam<<<blocks((long)sz[t]), 256, 0, h->stream>>>(s.w + o, s.m + o, s.v + o, s.g + o,
-                                                                   t < 4 ? s.wb + o : nullptr, (long)sz[t], lr_t, b1, b2,
-                                                                   c1, c2, eps);
-            }
-            if (cudaGetLastError() != cudaSuccess) {
-                rc = LBMGPU_E_CUDA;
-                break;
-            }
+            run(k_adam, blocks(kNParams), 256, s.w, s.m, s.v, s.g, s.wb, (long)kNParams, (long)off_w(4), lr_t, b1, b2, c1,
+                c2, eps);
+            if (rc) break;
             sum_n += (long)nb * kSurOut;
             s.train_steps += 1;
         }
@@ -1343,25 +1437,6 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
         for (long q = 0; q < (long)nparts * bi; ++q) sum_se += parts[q];
         epoch_loss = sum_n ? sum_se / sum_n : 0.0;
     }
-    cudaFree(idx);
-    cudaFree(Xb);
-    cudaFree(Yb);
-    cudaFree(vb);
-    cudaFree(H1);
-    cudaFree(H2);
-    cudaFree(H3);
-    cudaFree(Z1);
-    cudaFree(Z2);
-    cudaFree(Z3);
-    cudaFree(C);
-    cudaFree(dA);
-    cudaFree(dZ);
-    cudaFree(dZb);
-    cudaFree(T1);
-    cudaFree(T2);
-    cudaFree(Wt);
-    cudaFree(part);
-    cudaFree(Gp);
     if (rc) return rc;
     s.trained = true;
     s.last_loss = epoch_loss;
@@ -1398,20 +1473,16 @@ int lbmgpu_surrogate_eval(lbmgpu_t *h, const float *x, long n, float *y) {
         k_sur_standardise<<<blocks(mpad), 256, 0, h->stream>>>(xd, n, mpad, s.nrm, X);
         rc = run_mlp(h, X, pd, mpad);
     }
-    std::vector<float> out;
-    if (!rc) {
-        out.resize((size_t)mpad * kSurOutPad);
-        if (cudaMemcpyAsync(out.data(), pd, out.size() * 4, cudaMemcpyDeviceToHost, h->stream) ||
+    if (!rc) {  // the real outputs of the rows, packed where the inputs were (12 floats a row, 10 needed)
+        k_sur_pack<<<blocks(n * kSurOut), 256, 0, h->stream>>>(pd, n, xd);
+        if (cudaGetLastError() || cudaMemcpyAsync(y, xd, (size_t)n * kSurOut * 4, cudaMemcpyDeviceToHost, h->stream) ||
             cudaStreamSynchronize(h->stream))
             rc = LBMGPU_E_CUDA;
     }
     cudaFree(xd);
     cudaFree(X);
     cudaFree(pd);
-    if (rc) return rc;
-    for (long r = 0; r < n; ++r)
-        for (int q = 0; q < kSurOut; ++q) y[r * kSurOut + q] = out[r * kSurOutPad + q];
-    return LBMGPU_OK;
+    return rc;
 }
 
 int lbmgpu_surrogate_params(lbmgpu_t *h, float *buf, long n, int set) {
