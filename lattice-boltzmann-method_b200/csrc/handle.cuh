@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cstring>
 #include <thread>
 #include <vector>
 
@@ -178,6 +179,20 @@ void host_parallel_for(long n, const F &f, long min_items = 1024) {
     for (long t = 1; t < nt; ++t) th.emplace_back([&f, n, nt, t] { f(n * t / nt, n * (t + 1) / nt); });
     f(0L, n / nt);
     for (auto &x : th) x.join();
+}
+
+// Cells per chunk of a record transfer of `cells` cells: eight chunks or more, so that the host's copies
+// and the device's overlap, as far as the staging buffers and a chunk's fixed cost allow.
+inline long transfer_chunk(const lbmgpu *h, long cells) {
+    return std::min((long)h->stage_cells, std::max(8192L, (cells + 7) / 8));
+}
+
+// memcpy by host threads.
+inline void host_copy(void *dst, const void *src, size_t bytes) {
+    host_parallel_for((long)((bytes + 4095) / 4096), [&](long lo, long hi) {
+        const size_t a = (size_t)lo * 4096, b = std::min(bytes, (size_t)hi * 4096);
+        std::memcpy(static_cast<char *>(dst) + a, static_cast<const char *>(src) + a, b - a);
+    }, 256);
 }
 
 // Whether host memory at p is page-locked (registered or allocated by CUDA).

@@ -42,20 +42,20 @@ struct VtkSrc {
     UnitsF U;
 };
 
-// One cell's values into the arrays of the VTK file's appended data (cell data only),
-// each array at its offset in `out`, cells in x-fastest order.
-__global__ void k_vtk_pack(VtkSrc S, float *__restrict__ out) {
-    const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= S.ncell) return;
-    int i, j, k;
-    cell_ijk(n, S.si, S.sj, i, j, k);
-    const long o = ((long)k * S.Ny + j) * S.Nx + i, N = S.ncell;
+// The values of the cells o0 .. o1-1 in the file's x-fastest order: each array's part of these cells in
+// turn, N = o1 - o0 values per component.
+__global__ void k_vtk_pack(VtkSrc S, long o0, long o1, float *__restrict__ out) {
+    const long N = o1 - o0, o = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= N) return;
+    const unsigned q = (unsigned)(o0 + o), qj = q / (unsigned)S.Nx, i = q - qj * (unsigned)S.Nx, k = qj / (unsigned)S.Ny,
+                   j = qj - k * (unsigned)S.Ny;
+    const long n = (long)i * S.si + (long)j * S.sj + k, nc = S.ncell;
     const bool si = S.flags & LBMGPU_VTK_SI;
     const double *R = S.rec;
     const bool mc = S.ns > 0;
-    const double rho = R[(mc ? RM_RHO : M_RHO) * N + n];
-    const double u = R[(mc ? RM_U : M_U) * N + n], v = R[(mc ? RM_V : M_V) * N + n], w = R[(mc ? RM_W : M_W) * N + n];
-    const double T = R[(mc ? RM_T : M_T) * N + n], p = R[(mc ? RM_P : M_P) * N + n];
+    const double rho = R[(mc ? RM_RHO : M_RHO) * nc + n];
+    const double u = R[(mc ? RM_U : M_U) * nc + n], v = R[(mc ? RM_V : M_V) * nc + n], w = R[(mc ? RM_W : M_W) * nc + n];
+    const double T = R[(mc ? RM_T : M_T) * nc + n], p = R[(mc ? RM_P : M_P) * nc + n];
     out[o] = si ? si_rho(S.U, (float)rho) : (float)rho;
     out[N + 3 * o] = si ? si_u(S.U, (float)u) : (float)u;
     out[N + 3 * o + 1] = si ? si_u(S.U, (float)v) : (float)v;
@@ -64,12 +64,12 @@ __global__ void k_vtk_pack(VtkSrc S, float *__restrict__ out) {
     out[5 * N + o] = si ? si_temp(S.U, (float)T) : (float)T;
     out[6 * N + o] = si ? si_p(S.U, (float)p) : (float)p;
     if (!mc) return;
-    const double hrr = R[RM_HRR * N + n];
+    const double hrr = R[RM_HRR * nc + n];
     out[7 * N + o] = si ? si_hrr(S.U, (float)hrr) : (float)hrr;
     for (int a = 0; a < S.ns; ++a) {
-        const double ra = R[(long)rs(a, RS_RHO) * N + n];
-        out[(8 + a) * N + o] = (S.flags & LBMGPU_VTK_MASSFRAC) ? (float)(ra / rho) : (float)R[(long)rs(a, RS_X) * N + n];
-        const double du = R[(long)rs(a, RS_UX) * N + n] - u;
+        const double ra = R[(long)rs(a, RS_RHO) * nc + n];
+        out[(8 + a) * N + o] = (S.flags & LBMGPU_VTK_MASSFRAC) ? (float)(ra / rho) : (float)R[(long)rs(a, RS_X) * nc + n];
+        const double du = R[(long)rs(a, RS_UX) * nc + n] - u;
         out[(8 + S.ns + a) * N + o] = si ? si_u(S.U, (float)du) : (float)du;
     }
 }
@@ -106,15 +106,42 @@ int lbmgpu_vtk_fields(lbmgpu_t *h, float *out, size_t n_out, int flags) {
     const size_t need = (size_t)(vtk_arrays(h) + 2) * nc;  // velocity is three arrays wide
     if (n_out < need) return LBMGPU_E_ARG;
     CK(cudaSetDevice(h->d.device));
-    float *dbuf = nullptr;
-    CK(cudaMallocAsync(reinterpret_cast<void **>(&dbuf), need * sizeof(float), h->stream));
-    VtkSrc S{h->mom[h->cur], h->type, nc, h->g.si, h->g.sj, h->g.Nx, h->g.Ny, h->g.Nz, h->ns, flags, h->U};
-    k_vtk_pack<<<grid_for(nc), kBlock, 0, h->stream>>>(S, dbuf);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out, dbuf, need * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
-    cudaFreeAsync(dbuf, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    return e == cudaSuccess ? LBMGPU_OK : cuda_fail(e);
+    // piece by piece through the staging buffer and the two bounce buffers: while host threads place one
+    // piece's parts of the arrays, the device packs and copies the next
+    const int arrays = vtk_arrays(h);  // values per cell; the room for two more is cleared
+    const VtkSrc S{h->mom[h->cur], h->type, nc, h->g.si, h->g.sj, h->g.Nx, h->g.Ny, h->g.Nz, h->ns, flags, h->U};
+    const long fit = (long)(h->stage_bytes / (arrays * sizeof(float)));
+    const long step = std::max(1L, std::min(fit, std::max(16384L, (nc + 7) / 8)));
+    auto issue = [&](long o0, char *dst) -> int {
+        const long o1 = std::min(nc, o0 + step);
+        k_vtk_pack<<<grid_for(o1 - o0), kBlock, 0, h->stream>>>(S, o0, o1, reinterpret_cast<float *>(h->stage));
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(dst, h->stage, (size_t)(o1 - o0) * arrays * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+        return 0;
+    };
+    int rc = issue(0, h->bounce);
+    if (rc) return rc;
+    for (long o0 = 0, q = 0; o0 < nc; o0 += step, ++q) {
+        const long o1 = std::min(nc, o0 + step), N = o1 - o0;
+        const float *const buf = reinterpret_cast<const float *>((q & 1) ? h->bounce2 : h->bounce);
+        CK(cudaStreamSynchronize(h->stream));  // piece q is in buf
+        if (o1 < nc) {
+            rc = issue(o1, (q & 1) ? h->bounce : h->bounce2);
+            if (rc) return rc;
+        }
+        // components of the arrays: density, velocity (3 per cell, interleaved), then one each; last the unused room
+        host_parallel_for(arrays - 1, [&](long lo, long hi) {
+            for (long a = lo; a < hi; ++a) {
+                if (a == arrays - 2) {
+                    std::memset(out + arrays * nc + 2 * o0, 0, (size_t)(2 * N) * sizeof(float));
+                    continue;
+                }
+                const long at = a < 2 ? a : a + 2, width = a == 1 ? 3 : 1;
+                std::memcpy(out + at * nc + width * o0, buf + at * N, (size_t)(width * N) * sizeof(float));
+            }
+        }, N >= 32768 ? 1 : arrays);
+    }
+    return LBMGPU_OK;
 }
 
 int lbmgpu_write_vtk(lbmgpu_t *h, const char *path, int dx, int flags) {

@@ -577,40 +577,64 @@ int lbmgpu_upload(lbmgpu_t *h, const void *mixture_aos, const void *const *speci
     const long nc = g.ncell;
     const size_t rs = h->mo.size;
     const char *host = static_cast<const char *>(mixture_aos);
-    // cell types and the per-cell classification, computed on the host once per upload
+    // cell types and the per-cell classification, by host threads, x-plane by x-plane: the flags and each
+    // plane's count of special cells, then their compact indices in cell order
     std::vector<int8_t> ty(nc);
-    for (long n = 0; n < nc; ++n) {
-        short t;
-        std::memcpy(&t, host + n * rs + h->mo.type, sizeof(short));
-        if (t < 0 || t > 9) return LBMGPU_E_ARG;
-        ty[n] = (int8_t)t;
-    }
-    std::vector<uint8_t> cf(nc, 0);
+    std::vector<uint8_t> cf(nc, 0), bad(g.Nx, 0);
     std::vector<int> bidh(nc, -1);
-    std::vector<long> blh;
-    long nb = 0;
-    for (int i = 0; i < g.Nx; ++i)
-        for (int j = 0; j < g.Ny; ++j)
-            for (int k = 0; k < g.Nz; ++k) {
-                const long n = (long)i * g.si + (long)j * g.sj + k;
-                if (ty[n] != T_F) continue;
-                if (i == 0 || j == 0 || k == 0 || i == g.Nx - 1 || j == g.Ny - 1 || k == g.Nz - 1)
-                    return LBMGPU_E_ARG;  // a fluid cell on the outermost layer has no ghost neighbour
-                // special: a boundary cell upstream (solid, adiabatic, free-slip, inflow,
-                // outflow); the others stream with the branch-free periodic pull
-                uint8_t c = CF_FLUID;
-                for (int l = 0; l < 27; ++l) {
-                    const long s = n - (long)cx(l) * g.si - (long)cy(l) * g.sj - cz(l);
-                    const int t = ty[s];
-                    if (t == T_S || t == T_A || t == T_FS || t == T_I || t == T_O || t == T_I_C || t == T_O_C)
-                        c |= CF_SPECIAL;
-                }
-                if (c & CF_SPECIAL) {
-                    bidh[n] = (int)nb++;
-                    blh.push_back(n);
-                }
-                cf[n] = c;
+    std::vector<long> first(g.Nx, 0);
+    const long planes = std::max(1L, 16384 / g.si);  // x-planes worth a thread
+    host_parallel_for(g.Nx, [&](long lo, long hi) {
+        for (long i = lo; i < hi; ++i)
+            for (long n = i * g.si; n < (i + 1) * g.si; ++n) {
+                short t;
+                std::memcpy(&t, host + n * rs + h->mo.type, sizeof(short));
+                if (t < 0 || t > 9) bad[i] = 1;
+                ty[n] = (int8_t)t;
             }
+    }, planes);
+    for (int i = 0; i < g.Nx; ++i)
+        if (bad[i]) return LBMGPU_E_ARG;
+    host_parallel_for(g.Nx, [&](long lo, long hi) {
+        for (long i = lo; i < hi; ++i)
+            for (int j = 0; j < g.Ny; ++j)
+                for (int k = 0; k < g.Nz; ++k) {
+                    const long n = i * g.si + (long)j * g.sj + k;
+                    if (ty[n] != T_F) continue;
+                    if (i == 0 || j == 0 || k == 0 || i == g.Nx - 1 || j == g.Ny - 1 || k == g.Nz - 1) {
+                        bad[i] = 1;  // a fluid cell on the outermost layer has no ghost neighbour
+                        continue;
+                    }
+                    // special: a boundary cell upstream (solid, adiabatic, free-slip, inflow,
+                    // outflow); the others stream with the branch-free periodic pull
+                    uint8_t c = CF_FLUID;
+                    for (int l = 0; l < 27; ++l) {
+                        const int t = ty[n - (long)cx(l) * g.si - (long)cy(l) * g.sj - cz(l)];
+                        if (t == T_S || t == T_A || t == T_FS || t == T_I || t == T_O || t == T_I_C || t == T_O_C)
+                            c |= CF_SPECIAL;
+                    }
+                    if (c & CF_SPECIAL) ++first[i];
+                    cf[n] = c;
+                }
+    }, planes);
+    long nb = 0;
+    for (int i = 0; i < g.Nx; ++i) {
+        if (bad[i]) return LBMGPU_E_ARG;
+        const long in_plane = first[i];
+        first[i] = nb;
+        nb += in_plane;
+    }
+    std::vector<long> blh(nb);
+    host_parallel_for(g.Nx, [&](long lo, long hi) {
+        for (long i = lo; i < hi; ++i) {
+            long b = first[i];
+            for (long n = i * g.si; n < (i + 1) * g.si; ++n)
+                if (cf[n] & CF_SPECIAL) {
+                    bidh[n] = (int)b;
+                    blh[b++] = n;
+                }
+        }
+    }, planes);
     // (re)size the boundary store
     if (nb != h->nb || !h->bst[0]) {
         for (int b = 0; b < 2; ++b) {
@@ -638,9 +662,24 @@ int lbmgpu_upload(lbmgpu_t *h, const void *mixture_aos, const void *const *speci
     CK(cudaMemcpyAsync(h->cflag, cf.data(), nc, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->bid, bidh.data(), nc * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     h->cur = 0;
-    for (long n0 = 0; n0 < nc; n0 += (long)h->stage_cells) {
-        const long n1 = std::min<long>(nc, n0 + (long)h->stage_cells);
-        CK(cudaMemcpyAsync(h->stage, host + n0 * rs, (n1 - n0) * rs, cudaMemcpyHostToDevice, h->stream));
+    // page-locked records are copied directly; host threads fill one bounce buffer with pageable ones
+    // while the other's copy is under way (fork and join mark them: no step is running)
+    const bool pinned = host_pinned(host);
+    const long step = pinned ? (long)h->stage_cells : transfer_chunk(h, nc);
+    const cudaEvent_t copied[2] = {h->fork, h->join};
+    if (!pinned) CK(cudaStreamSynchronize(h->stream));  // the bounce buffers' earlier copies have gone
+    long chunk = 0;
+    for (long n0 = 0; n0 < nc; n0 += step, ++chunk) {
+        const long n1 = std::min<long>(nc, n0 + step);
+        if (pinned) {
+            CK(cudaMemcpyAsync(h->stage, host + n0 * rs, (n1 - n0) * rs, cudaMemcpyHostToDevice, h->stream));
+        } else {
+            char *const bounce = chunk & 1 ? h->bounce2 : h->bounce;
+            if (chunk >= 2) CK(cudaEventSynchronize(copied[chunk & 1]));
+            host_copy(bounce, host + n0 * rs, (n1 - n0) * rs);
+            CK(cudaMemcpyAsync(h->stage, bounce, (n1 - n0) * rs, cudaMemcpyHostToDevice, h->stream));
+            CK(cudaEventRecord(copied[chunk & 1], h->stream));
+        }
         EvPair ep{};
         ev_begin(h, K_OTHER, ep);
         k_sc_unpack<<<grid_for(n1 - n0), kBlock, 0, h->stream>>>(g, h->P, h->mo, h->stage, n0, n1, h->cflag,
@@ -730,50 +769,67 @@ int lbmgpu_download(lbmgpu_t *h, void *mixture_aos, void *const *species_aos) {
     CK(cudaStreamSynchronize(h->stream));
     const int c = h->cur;
     const long mof[6] = {h->mo.rho, h->mo.u, h->mo.v, h->mo.w, h->mo.temp, h->mo.p};
-    for (long n0 = 0; n0 < nc; n0 += (long)h->stage_cells) {
-        const long n1 = std::min<long>(nc, n0 + (long)h->stage_cells);
+    // chunk k is packed on the device and copied into bounce buffer k % 2; while host threads merge chunk
+    // k, the device packs and copies chunk k + 1 into the other buffer
+    const long step = transfer_chunk(h, nc);
+    auto issue = [&](long n0, char *dst) -> int {
+        const long n1 = std::min<long>(nc, n0 + step);
         CK(cudaMemsetAsync(h->stage, 0, (size_t)(n1 - n0) * rs, h->stream));  // zero padding bytes
         EvPair ep{};
         ev_begin(h, K_OTHER, ep);
         const unsigned gb = grid_for(n1 - n0);
+        auto pack = [&](auto kernel) {
+            kernel<<<gb, kBlock, 0, h->stream>>>(g, h->P, h->mo, h->stage, n0, n1, h->type, h->cflag, h->bid, h->pop[c],
+                                                 h->mom[c], h->bst[c], h->nb);
+        };
         if (h->pack_mode == PK_STEPPED)
-            k_sc_pack<PK_STEPPED><<<gb, kBlock, 0, h->stream>>>(g, h->P, h->mo, h->stage, n0, n1, h->type, h->cflag,
-                                                                h->bid, h->pop[c], h->mom[c], h->bst[c], h->nb);
+            pack(k_sc_pack<PK_STEPPED>);
         else if (h->pack_mode == PK_INIT)
-            k_sc_pack<PK_INIT><<<gb, kBlock, 0, h->stream>>>(g, h->P, h->mo, h->stage, n0, n1, h->type, h->cflag,
-                                                             h->bid, h->pop[c], h->mom[c], h->bst[c], h->nb);
+            pack(k_sc_pack<PK_INIT>);
         else
-            k_sc_pack<PK_UPLOADED><<<gb, kBlock, 0, h->stream>>>(g, h->P, h->mo, h->stage, n0, n1, h->type,
-                                                                 h->cflag, h->bid, h->pop[c], h->mom[c], h->bst[c],
-                                                                 h->nb);
+            pack(k_sc_pack<PK_UPLOADED>);
         ev_end(h, ep);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(h->bounce, h->stage, (n1 - n0) * rs, cudaMemcpyDeviceToHost, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
-        // merge: fluid cells take the whole record except the type; the others only
-        // their stored moments (ghost populations are not represented on the device)
-        for (long n = n0; n < n1; ++n) {
-            const char *srec = h->bounce + (n - n0) * rs;
-            char *drec = host + n * rs;
-            if (ty[n] == T_F && h->pack_mode == PK_STEPPED) {
-                // every field of a stepped fluid cell was produced: the whole record but the type
-                short t;
-                std::memcpy(&t, drec + h->mo.type, sizeof(short));
-                std::memcpy(drec, srec, rs);
-                std::memcpy(drec + h->mo.type, &t, sizeof(short));
-            } else {
-                for (int m = 0; m < 6; ++m) std::memcpy(drec + mof[m], srec + mof[m], sizeof(double));
-                if (ty[n] == T_F) {
-                    std::memcpy(drec + h->mo.f, srec + h->mo.f, 27 * sizeof(double));
-                    std::memcpy(drec + h->mo.g, srec + h->mo.g, 27 * sizeof(double));
-                    if (h->pack_mode == PK_INIT) {
-                        std::memcpy(drec + h->mo.p_tensor, srec + h->mo.p_tensor, 9 * sizeof(double));
-                        std::memcpy(drec + h->mo.rhoe, srec + h->mo.rhoe, sizeof(double));
+        CK(cudaMemcpyAsync(dst, h->stage, (n1 - n0) * rs, cudaMemcpyDeviceToHost, h->stream));
+        return 0;
+    };
+    int rc = issue(0, h->bounce);
+    if (rc) return rc;
+    for (long n0 = 0, q = 0; n0 < nc; n0 += step, ++q) {
+        const long n1 = std::min<long>(nc, n0 + step);
+        const char *const buf = (q & 1) ? h->bounce2 : h->bounce;
+        CK(cudaStreamSynchronize(h->stream));  // chunk q is in buf
+        if (n1 < nc) {
+            rc = issue(n1, (q & 1) ? h->bounce : h->bounce2);
+            if (rc) return rc;
+        }
+        // merge: fluid cells take the whole record except the type; the others only their stored
+        // moments (ghost populations are not represented on the device)
+        host_parallel_for(n1 - n0, [&](long lo, long hi) {
+            for (long n = n0 + lo; n < n0 + hi; ++n) {
+                const char *srec = buf + (n - n0) * rs;
+                char *drec = host + n * rs;
+                if (ty[n] == T_F && h->pack_mode == PK_STEPPED) {
+                    // every field of a stepped fluid cell was produced: the whole record but the type
+                    short t;
+                    std::memcpy(&t, drec + h->mo.type, sizeof(short));
+                    std::memcpy(drec, srec, rs);
+                    std::memcpy(drec + h->mo.type, &t, sizeof(short));
+                } else {
+                    for (int m = 0; m < 6; ++m) std::memcpy(drec + mof[m], srec + mof[m], sizeof(double));
+                    if (ty[n] == T_F) {
+                        std::memcpy(drec + h->mo.f, srec + h->mo.f, 27 * sizeof(double));
+                        std::memcpy(drec + h->mo.g, srec + h->mo.g, 27 * sizeof(double));
+                        if (h->pack_mode == PK_INIT) {
+                            std::memcpy(drec + h->mo.p_tensor, srec + h->mo.p_tensor, 9 * sizeof(double));
+                            std::memcpy(drec + h->mo.rhoe, srec + h->mo.rhoe, sizeof(double));
+                        }
                     }
                 }
             }
-        }
+        });
     }
+    CK(cudaStreamSynchronize(h->stream));
     return LBMGPU_OK;
 }
 

@@ -365,7 +365,7 @@ int mc_download_planes(lbmgpu *h, int i0, int i1, void *mix, void *const *specie
     char *hm = static_cast<char *>(mix);
     // chunk k is packed on the device and copied into bounce buffer k % 2; while the host
     // merges chunk k, the device packs and copies chunk k + 1 into the other buffer
-    const long step = (long)h->stage_cells;
+    const long step = transfer_chunk(h, c1 - c0);
     auto issue = [&](long n0, char *dst) -> int {
         const long n1 = std::min<long>(c1, n0 + step);
         const int rc = mc_by_ns(h->ns, [&](auto ops) { return decltype(ops)::pack(h, n0, n1, stepped); });

@@ -178,8 +178,15 @@ int upload_t(lbmgpu *h, const char *hm, const void *const *species, long c0, lon
     // page-locked caller memory is copied directly
     bool pinned = host_pinned(hm);
     for (int a = 0; a < h->ns; ++a) pinned = pinned && host_pinned(species[a]);
-    for (long n0 = c0; n0 < c1; n0 += (long)h->stage_cells) {
-        const long n1 = std::min<long>(c1, n0 + (long)h->stage_cells), cnt = n1 - n0;
+    // host threads fill one bounce buffer while the other's copy is under way; fork and join mark the two
+    // buffers' copies (no step is running during an upload)
+    const long step = pinned ? (long)h->stage_cells : transfer_chunk(h, c1 - c0);
+    const cudaEvent_t copied[2] = {h->fork, h->join};
+    if (!pinned) CK(cudaStreamSynchronize(h->stream));  // the bounce buffers' earlier copies have gone
+    long chunk = 0;
+    for (long n0 = c0; n0 < c1; n0 += step, ++chunk) {
+        const long n1 = std::min<long>(c1, n0 + step), cnt = n1 - n0;
+        char *const bounce = chunk & 1 ? h->bounce2 : h->bounce;
         if (pinned) {
             CK(cudaMemcpyAsync(h->stage, hm + (n0 - c0) * ms, cnt * ms, cudaMemcpyHostToDevice, h->stream));
             for (int a = 0; a < h->ns; ++a)
@@ -187,20 +194,20 @@ int upload_t(lbmgpu *h, const char *hm, const void *const *species, long c0, lon
                                    static_cast<const char *>(species[a]) + (n0 - c0) * ss, cnt * ss,
                                    cudaMemcpyHostToDevice, h->stream));
         } else {
-            CK(cudaStreamSynchronize(h->stream));  // the bounce buffer's previous chunk has gone
-            const long nb = (long)h->ns + 1;       // the mixture block, then each species' block
+            if (chunk >= 2) CK(cudaEventSynchronize(copied[chunk & 1]));  // the buffer's previous chunk has gone
+            const long nb = (long)h->ns + 1;  // the mixture block, then each species' block
             host_parallel_for(nb * 64, [&](long lo, long hi) {
                 for (long q = lo; q < hi; ++q) {
                     const long blk = q / 64, part = q % 64;
                     const size_t sz = blk == 0 ? ms : ss;
                     const char *src = blk == 0 ? hm : static_cast<const char *>(species[blk - 1]);
-                    char *dst = h->bounce + (blk == 0 ? 0 : cnt * ms + (size_t)(blk - 1) * cnt * ss);
+                    char *dst = bounce + (blk == 0 ? 0 : cnt * ms + (size_t)(blk - 1) * cnt * ss);
                     const long r0 = cnt * part / 64, r1 = cnt * (part + 1) / 64;
                     std::memcpy(dst + r0 * sz, src + (n0 - c0 + r0) * sz, (r1 - r0) * sz);
                 }
             }, 1);
-            CK(cudaMemcpyAsync(h->stage, h->bounce, cnt * (ms + (size_t)h->ns * ss), cudaMemcpyHostToDevice,
-                               h->stream));
+            CK(cudaMemcpyAsync(h->stage, bounce, cnt * (ms + (size_t)h->ns * ss), cudaMemcpyHostToDevice, h->stream));
+            CK(cudaEventRecord(copied[chunk & 1], h->stream));
         }
         EvPair ep{};
         ev_begin(h, K_OTHER, ep);
