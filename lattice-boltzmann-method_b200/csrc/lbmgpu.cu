@@ -57,7 +57,8 @@ __device__ __forceinline__ double fd_central(double sl, double sc, double sr, in
 // everything it needs -- its 27 populations, the record, the face terms and types -- before its
 // cell's flag is known (at the nearest interior cell), so a block waits for one round of memory
 // latency; one thread for both sets went through four (flag, record, f, g).
-// Measured: 150 x 121 x 113 cells 440 -> 349 us (970 B a cell: 5.7 TB/s), 64^3 68 -> 52 us.
+// Measured: 150 x 121 x 113 cells 440 -> 349 us (970 B a cell: 5.7 TB/s), 64^3 68 -> 52 us.  The energy
+// set's flux correction is the difference of two equilibria, rounded as one thread per cell rounded it.
 template <bool LOCAL>
 __global__ void __launch_bounds__(2 * kBlock, 2)
     k_sc_collide(ScGeom g, ScPhys P, const int8_t *__restrict__ type, const uint8_t *__restrict__ cflag,
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(2 * kBlock, 2)
 #pragma unroll
         for (int a = 0; a < 3; ++a) corr[a] = dt * (2 - om) / (2 * rho * om) * dQ[a];
         AxisF<double> F;
-        axis_feq(F, vel, theta, corr);
+        axis_feq_sc<LOCAL ? 0 : 1>(F, vel, theta, corr);
 #pragma unroll
         for (int l = 0; l < 27; ++l) d0[(long)l * nc] = (1.0 - om) * v[l] + om * feq_l(l, rho, F);
         return;
@@ -127,14 +128,15 @@ __global__ void __launch_bounds__(2 * kBlock, 2)
 #pragma unroll
     for (int a = 0; a < 3; ++a) dq[a] = S[a] + 0.5 * dt * vel[a] * dQ[a];
     AxisG<double> G;
-    axis_geq(G, Uint, theta, vel);
-    const double kq = 0.5 * (om1 - om);
+    axis_geq_sc<LOCAL ? 0 : 1>(G, Uint, theta, vel);
 #pragma unroll
     for (int l = 0; l < 27; ++l) {
-        const double gq = geq_l(l, rho, G);
+        const double gq = __dmul_rn(rho, geq_l(l, 1.0, G));
         double out = v[l] + om1 * (gq - v[l]);
-        if (csq(l) == 1)  // the flux correction acts along the six axes
-            out += kq * (cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2]));
+        if (csq(l) == 1) {  // the flux correction acts along the six axes
+            const double gs = gq + 0.5 * (cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2]));
+            out += (om - om1) * (gq - gs);
+        }
         d0[(long)l * nc] = out;
     }
 }
@@ -365,7 +367,7 @@ int launch_stream_moment(lbmgpu *h) {
         CK(cudaStreamWaitEvent(h->side, h->fork, 0));
         EvPair eb{};
         ev_begin(h, K_OTHER, eb, h->side);
-        k_sc_special<<<(unsigned)((h->nb + kScSpCells - 1) / kScSpCells), 2 * kScSpCells, 0, h->side>>>(
+        k_sc_special<<<(unsigned)((h->nb + kScSpBlock - 1) / kScSpBlock), kScSpBlock, 0, h->side>>>(
             h->g, h->P, h->type, h->blist, h->pop[x], h->mom[c], h->mom[x], h->bst[c], h->bst[x], h->nb, h->status);
         ev_end(h, eb, h->side);
         CK(cudaGetLastError());

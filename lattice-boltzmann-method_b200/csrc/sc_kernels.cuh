@@ -97,6 +97,33 @@ __device__ __forceinline__ int pull_at(const PullSrc &s, int l) {
     return s.X[cidx(cx(l))] + s.Y[cidx(cy(l))] + s.Z[cidx(cz(l))];
 }
 
+// The per-axis factors with u_a^2 rounded by itself before theta is added, for the axes from FIRST on (a
+// product with one use only would be fused into the sum).  Both population sets, in their own threads, and
+// the steps after an upload and later ones then round as they did in one thread per cell, to the bit: a
+// velocity component that decays to 1e-7 of the sound speed keeps only nine digits through any other
+// rounding.
+template <int FIRST>
+__device__ __forceinline__ void axis_feq_sc(AxisF<double> &F, const double u[3], double theta, const double corr[3]) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double z = theta + (a < FIRST ? u[a] * u[a] : __dmul_rn(u[a], u[a])) + corr[a];
+        F.v[a][0] = 1.0 - z;
+        F.v[a][1] = (u[a] + z) * 0.5;
+        F.v[a][2] = (-u[a] + z) * 0.5;
+    }
+}
+template <int FIRST>
+__device__ __forceinline__ void axis_geq_sc(AxisG<double> &G, double U, double theta, const double u[3]) {
+    axis_geq(G, U, theta, u);
+#pragma unroll
+    for (int a = FIRST; a < 3; ++a) {
+        const double z = theta + __dmul_rn(u[a], u[a]);
+        G.P[a][0] = 1.0 - z;
+        G.P[a][1] = (u[a] + z) * 0.5;
+        G.P[a][2] = (-u[a] + z) * 0.5;
+    }
+}
+
 // Sums of the moments of one cell: rho, j, P (upper triangle), rhoe, q.
 struct ScSums {
     double rho, j[3], P[6], re, q[3];

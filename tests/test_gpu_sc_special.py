@@ -1,4 +1,4 @@
-"""The single-component boundary cells' kernel (csrc/sc_special.cuh: two warps per 32 listed cells)
+"""The single-component boundary cells' kernel (csrc/sc_special.cuh: blocks of 32 listed cells)
 and the collision's two halves against the C oracle, at lattice sizes around a block's 32 cells and
 128 cells, with inflow, outflow, solid, adiabatic and free-slip cells.  FP64 on both sides; the
 device's sums and factors differ from the oracle's by rounding: 1e-12 of each field's magnitude (the
