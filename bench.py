@@ -372,14 +372,14 @@ def run_reference(args, dist):
 def mc_bytes(kernel, pop_bytes, reaction=False):
     """Algorithmic bytes per fluid cell of one multicomponent launch (9 species): every
     population (270 planes of `pop_bytes`) read once and, by the update, written once;
-    the FP64 record, parameter and sum planes each kernel must read or write once per cell.
+    the FP64 record and parameter planes each kernel must read or write once per cell.
       k_mc_relax : 270 populations in and out; per species rho_a, the 3 face terms and
                    the parameters om_a, F_a (3) [, drho_a]; shared u (3), T, rho; the
                    energy set's 7 parameters -> 9 * (4 + 4) + 5 + 7 = 84 planes [+ 9]
-      k_mc_gather: 270 populations pulled, 91 sum planes written (per species rho_a, j_a,
-                   its P-tensor share; the energy sum)
-      k_mc_solve : the 91 sum planes, 21 record planes (rho, T, p, rho_a, X_a) and the 36
-                   D_ab read, 88 record planes written
+      k_mc_gather, k_mc_solve : moments split at 91 planes of sums (per species rho_a, j_a, its
+                   P-tensor share; the energy sum), which the one writes and the other reads
+                   beside 21 record planes and the 36 D_ab, 88 record planes written; the
+                   device's own split is step_bytes below
       k_mc_props : 58 record planes of the cell, 86 parameter planes written (49 + the 36
                    D_ab + R/W) [+ HRR]
       k_mc_eflux : 53 record planes of the cell (rho, u, T, p, rho_a, u_a, the P tensor, the
@@ -393,6 +393,21 @@ def mc_bytes(kernel, pop_bytes, reaction=False):
     if kernel == "k_mc_solve":
         return (91 + 21 + 36 + 88) * 8
     return 270 * pop_bytes + 91 * 8  # k_mc_gather
+
+
+def step_bytes(kernel, pop_bytes, reaction=False):
+    """mc_bytes of the kernels a step launches, with the moments split where the device splits them:
+      k_mc_gather : 270 populations pulled, 47 record planes written (rho, u, P, rhoE; per
+                    species rho_a, j_a)
+      k_mc_diffuse: rho, u, T, p, rho_a, j_a and the 36 D_ab read, u_a written
+      k_mc_thermo : rho, u, rhoE, P, T, rho_a, u_a read, T, p, X_a and the 30 face terms written"""
+    if kernel == "k_mc_gather":
+        return 270 * pop_bytes + 47 * 8
+    if kernel == "k_mc_diffuse":
+        return (6 + 36 + 36 + 27) * 8
+    if kernel == "k_mc_thermo":
+        return (12 + 36 + 2 + 9 + 30) * 8
+    return mc_bytes(kernel, pop_bytes, reaction)
 
 
 MC_SHAPES = {"mix": "periodic", "react": "periodic", "inflow": "TYPE_I_C inflow / TYPE_O_C outflow in x, periodic y z",
@@ -615,11 +630,11 @@ def run_ours_mc(args, dist):
             sur.update(surrogate_vs_plain(lat, mix, sp, args.compare, sur["refresh_s"], sur_cap))
     lat.close()
     avg = {"k_mc_relax": kms[0] / max(launches[0], 1), "k_mc_gather": kms[1] / max(launches[1], 1),
-           "k_mc_solve": kms[5] / max(launches[5], 1), "k_mc_props": kms[3] / max(launches[3], 1),
+           "k_mc_diffuse + k_mc_thermo": kms[5] / max(launches[5], 1), "k_mc_props": kms[3] / max(launches[3], 1),
            "k_mc_eflux": kms[6] / max(launches[6], 1)}
     hbm_kernels = ("k_mc_relax", "k_mc_gather")
     dom = max(hbm_kernels, key=avg.get)  # the dominant population-moving kernel
-    alg = mc_bytes(dom, pop_bytes, reaction) * ncell
+    alg = step_bytes(dom, pop_bytes, reaction) * ncell
     peak, peak_kind = peaks()
     achieved = alg / (avg[dom] * 1e-3) / 1e9
 
@@ -667,7 +682,7 @@ def run_ours_mc(args, dist):
                    "storage": ("FP32 populations (shifted), FP64 records; transport properties in FP32, the "
                                "chemistry, moment solve and temperature recovery in FP64") if pop_bytes == 4
                    else "FP64"},
-        "hbm_gbs_step": ncell * sum(mc_bytes(k, pop_bytes, reaction) for k in ("k_mc_relax", "k_mc_gather", "k_mc_solve", "k_mc_props", "k_mc_eflux"))
+        "hbm_gbs_step": ncell * sum(step_bytes(k, pop_bytes, reaction) for k in ("k_mc_relax", "k_mc_gather", "k_mc_diffuse", "k_mc_thermo", "k_mc_props", "k_mc_eflux"))
         / (ms / args.steps * 1e-3) / 1e9,
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
@@ -1121,7 +1136,7 @@ def run_ours_turb(args, dist):
     launches, kms = lat.kernel_times()
     lat.profile(False)
     names = {0: "k_mc_relax", 1: "k_mc_gather", 2: "k_mc_special (+ other; slabs: + halo pack/unpack)",
-             3: "k_mc_props", 5: "k_mc_solve", 6: "k_mc_eflux", 7: "k_mc_chem"}
+             3: "k_mc_props", 5: "k_mc_diffuse + k_mc_thermo", 6: "k_mc_eflux", 7: "k_mc_chem"}
     per_step = {names[k]: kms[k] / kk for k in names}
     prof_step = sum(per_step.values())
     step_ms = ms / args.steps
@@ -1130,13 +1145,13 @@ def run_ours_turb(args, dist):
     achieved = alg_step * ncell / (step_ms * 1e-3) / 1e9
     kern = {}
     case = f"turb_{args.precision}"
-    step_kernels = ("k_mc_props", "k_mc_chem", "k_mc_eflux", "k_mc_relax", "k_mc_special", "k_mc_gather", "k_mc_solve")
+    step_kernels = ("k_mc_props", "k_mc_chem", "k_mc_eflux", "k_mc_relax", "k_mc_special", "k_mc_gather", "k_mc_diffuse", "k_mc_thermo")
     # the boundary kernel's cells are the two planes next to the outflow faces (2 N^2 per box)
     parts = [ncu_traffic(name, 2 * N * N if name == "k_mc_special" else ncell, case)
              for name in step_kernels]
     step_traffic = sum(parts) if all(p_ is not None for p_ in parts) else None
     for k, name in ((0, "k_mc_relax"), (1, "k_mc_gather")):
-        alg = mc_bytes(name, pop_bytes, True) * ncell
+        alg = step_bytes(name, pop_bytes, True) * ncell
         t = kms[k] / max(launches[k], 1)
         kern[name] = {"alg_bytes_per_launch": alg, "mean_launch_ms": t, "achieved_gbs": alg / (t * 1e-3) / 1e9,
                       "frac": alg / (t * 1e-3) / 1e9 / peak, "traffic": ncu_traffic(name, ncell, case)}
