@@ -174,11 +174,16 @@ void host_parallel_for(long n, const F &f, long min_items = 1024) {
         f(0L, n);
         return;
     }
-    std::vector<std::thread> th;
-    th.reserve(nt - 1);
-    for (long t = 1; t < nt; ++t) th.emplace_back([&f, n, nt, t] { f(n * t / nt, n * (t + 1) / nt); });
+    std::thread th[32];
+    long t = 1;
+    try {
+        for (; t < nt; ++t) th[t] = std::thread([&f, n, nt, t] { f(n * t / nt, n * (t + 1) / nt); });
+    } catch (...) {  // no more threads to be had: this one takes the ranges that are left
+    }
     f(0L, n / nt);
-    for (auto &x : th) x.join();
+    for (; t < nt; ++t) f(n * t / nt, n * (t + 1) / nt);
+    for (auto &x : th)
+        if (x.joinable()) x.join();
 }
 
 // Cells per chunk of a record transfer of `cells` cells: eight chunks or more, so that the host's copies
