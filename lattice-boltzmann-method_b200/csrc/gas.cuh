@@ -273,6 +273,68 @@ GAS_HD int T_from_u_n(const Tables &t, const double *Y, double u, double T0, dou
     return -1;
 }
 
+// The stopping rule of the moments' temperature iteration: a step dT from T_was to T below 1e-14 T, or one
+// below 1e-8 T between two temperatures of the same polynomial range of every species.  The iteration is
+// Newton's with the exact derivative, so within one range the step after the latter is below 1e-16 T and
+// need not be taken; across a range's end c_p jumps, and a last step of 1e-8 T would leave that jump's
+// share of it as the error.
+template <int NS>
+GAS_HD bool newton_done(const double *T_mid, double T_was, double dT, double T) {
+    if (!(fabs(dT) <= 1e-8 * T)) return false;
+    if (fabs(dT) <= 1e-14 * T) return true;
+    for (int k = 0; k < NS; ++k)
+        if ((T_was < T_mid[k]) != (T < T_mid[k])) return false;
+    return true;
+}
+
+// The NASA-7 coefficients of the temperature iteration on their own (a block's shared memory).
+template <int NS>
+struct ThermoTab {
+    double h[NS][2][6], c[NS][2][5], T_mid[NS], invW[NS];
+    // entries first, first + step, ...
+    GAS_HD void fill(const Tables &t, int first, int step) {
+        for (int i = first; i < NS * 12; i += step) h[i / 12][i / 6 % 2][i % 6] = t.hcoef[i / 12][i / 6 % 2][i % 6];
+        for (int i = first; i < NS * 10; i += step)
+            c[i / 10][i / 5 % 2][i % 5] = (i / 5 % 2 ? t.m.nasa_hi : t.m.nasa_lo)[i / 10][i % 5];
+        for (int i = first; i < NS; i += step) {
+            T_mid[i] = t.m.T_mid[i];
+            invW[i] = t.invW[i];
+        }
+    }
+};
+
+// T_from_u_n, or (FAST) T_from_u_fast, from the table, with the rule above.
+template <int NS, bool FAST>
+GAS_HD int T_from_u_tab(const ThermoTab<NS> &s, const double *Y, double u, double T0, double &T) {
+    T = T0 > 0 ? T0 : 300.0;
+    for (int it = 0; it < 100; ++it) {
+        const double invT = FAST ? 1.0 / T : 0.0, T_was = T;
+        double e = 0.0, c = 0.0;
+#pragma unroll
+        for (int k = 0; k < NS; ++k) {
+            const int r = T < s.T_mid[k] ? 0 : 1;
+            const double *h = s.h[k][r], *a = s.c[k][r];
+            const double hRT = h[0] + T * (h[1] + T * (h[2] + T * (h[3] + T * h[4]))) + (FAST ? h[5] * invT : h[5] / T);
+            const double cpR = a[0] + T * (a[1] + T * (a[2] + T * (a[3] + T * a[4])));
+            e += Y[k] * (hRT - 1.0) * s.invW[k];
+            c += Y[k] * (cpR - 1.0) * s.invW[k];
+        }
+        double dT;
+        if (FAST) {
+            dT = -(e * kR * T - u) / (c * kR);
+        } else {
+            const double f = e * kR * T - u;
+            const double cv = c * kR;
+            dT = -f / cv;
+        }
+        if (dT > 500.0) dT = 500.0;
+        if (dT < -0.5 * T) dT = -0.5 * T;
+        T += dT;
+        if (newton_done<NS>(s.T_mid, T_was, dT, T)) return it + 1;
+    }
+    return -1;
+}
+
 // ---- transport: kinetic theory (evaluated at setup only) ---------------------------
 inline double species_visc_kt(const Tables &t, int k, double T) {
     return t.visc_pref[k] * sqrt(T) / omega22(T / t.eps[k], t.delta[k]);

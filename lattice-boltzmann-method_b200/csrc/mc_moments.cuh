@@ -137,65 +137,15 @@ __global__ void __launch_bounds__(128, 3) k_mc_diffuse(McArgsT<S, double> A) {
         for (int d = 0; d < 3; ++d) put(A, R, rs(a, RS_UX + d), n, us[a][d]);
 }
 
-// The NASA-7 coefficients of the temperature iteration in shared memory.
-template <int NS>
-struct ThermoTab {
-    double h[NS][2][6], c[NS][2][5], T_mid[NS], invW[NS];
-};
-template <int NS>
-__device__ __forceinline__ void thermo_load(ThermoTab<NS> &s, const gas::Tables &t) {
-    for (int i = threadIdx.x; i < NS * 12; i += blockDim.x) s.h[i / 12][i / 6 % 2][i % 6] = t.hcoef[i / 12][i / 6 % 2][i % 6];
-    for (int i = threadIdx.x; i < NS * 10; i += blockDim.x)
-        s.c[i / 10][i / 5 % 2][i % 5] = (i / 5 % 2 ? t.m.nasa_hi : t.m.nasa_lo)[i / 10][i % 5];
-    for (int i = threadIdx.x; i < NS; i += blockDim.x) {
-        s.T_mid[i] = t.m.T_mid[i];
-        s.invW[i] = t.invW[i];
-    }
-    __syncthreads();
-}
-
-// T_from_u_n / T_from_u_fast from the shared table.  The iteration is Newton's with the exact
-// derivative: once a step is below kNewtonTol of T, the step after it would be below 1e-16 T.
-constexpr double kNewtonTol = 1e-8;
-template <int NS, bool FAST>
-__device__ __forceinline__ int thermo_T_from_u(const ThermoTab<NS> &s, const double *Y, double u, double T0, double &T) {
-    T = T0 > 0 ? T0 : 300.0;
-    for (int it = 0; it < 100; ++it) {
-        const double invT = FAST ? 1.0 / T : 0.0;
-        double e = 0.0, c = 0.0;
-#pragma unroll
-        for (int k = 0; k < NS; ++k) {
-            const int r = T < s.T_mid[k] ? 0 : 1;
-            const double *h = s.h[k][r], *a = s.c[k][r];
-            const double hRT = h[0] + T * (h[1] + T * (h[2] + T * (h[3] + T * h[4]))) + (FAST ? h[5] * invT : h[5] / T);
-            const double cpR = a[0] + T * (a[1] + T * (a[2] + T * (a[3] + T * a[4])));
-            e += Y[k] * (hRT - 1.0) * s.invW[k];
-            c += Y[k] * (cpR - 1.0) * s.invW[k];
-        }
-        double dT;
-        if (FAST) {
-            dT = -(e * gas::kR * T - u) / (c * gas::kR);
-        } else {
-            const double f = e * gas::kR * T - u;
-            const double cv = c * gas::kR;
-            dT = -f / cv;
-        }
-        if (dT > 500.0) dT = 500.0;
-        if (dT < -0.5 * T) dT = -0.5 * T;
-        T += dT;
-        if (fabs(dT) <= kNewtonTol * T) return it + 1;
-    }
-    return -1;
-}
-
 // Temperature from the internal energy (setState_UV, lbm-moment.cpp:346-368), pressure, mole
 // fractions and the face terms of every interior cell.
 template <int NS, typename S>
 __global__ void __launch_bounds__(128, 5) k_mc_thermo(McArgsT<S, double> A) {
     constexpr bool fast = sizeof(S) == sizeof(float);
-    __shared__ ThermoTab<NS> tab;
+    __shared__ gas::ThermoTab<NS> tab;  // the temperature iteration's coefficients
     const gas::Tables &t = *A.tab;
-    thermo_load(tab, t);
+    tab.fill(t, threadIdx.x, blockDim.x);
+    __syncthreads();
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= A.ncell) return;
     lbmh::step_begin();
@@ -234,7 +184,7 @@ __global__ void __launch_bounds__(128, 5) k_mc_thermo(McArgsT<S, double> A) {
     const double vol = 1.0 / (double)si_rho(A.U, (float)rho);
     const double rho_n_si = 1.0 / vol;
     double Tn;
-    if (thermo_T_from_u<NS, fast>(tab, Y, u_si, T_si, Tn) < 0) atomic_status(A.status, LBMGPU_ST_NEWTON);
+    if (gas::T_from_u_tab<NS, fast>(tab, Y, u_si, T_si, Tn) < 0) atomic_status(A.status, LBMGPU_ST_NEWTON);
     const double Pn = rho_n_si * gas::kR * Tn / Wn;
     const double Tl = u_temp(A.U, (float)Tn);
     put(A, R, RM_T, n, Tl);

@@ -94,11 +94,13 @@ __device__ __forceinline__ double sp_mass_fractions(SpBlock<NS> &B, const gas::T
 }
 
 // T_from_u / T_from_u_fast of the cells that are `on`, with the thread's species' share per
-// iteration; the block iterates until its last cell has converged.
-template <int NS, bool FAST>
+// iteration; the block iterates until its last cell has converged: by the moments' rule
+// (MOMENTS, gas::newton_done), or to the local state's 1e-9.
+template <int NS, bool FAST, bool MOMENTS>
 __device__ __forceinline__ int sp_T_from_u(SpBlock<NS> &B, const gas::Tables &t, double Y, double u, double T0,
-                                           double rtol, int maxit, bool on, double &T) {
+                                           bool on, double &T) {
     T = T0 > 0 ? T0 : 300.0;
+    constexpr int maxit = 100;
     int it_used = on ? -1 : 0;
     const int a = B.set < NS ? B.set : NS - 1;
     for (int it = 0; it <= maxit; ++it) {
@@ -123,8 +125,9 @@ __device__ __forceinline__ int sp_T_from_u(SpBlock<NS> &B, const gas::Tables &t,
         }
         if (dT > 500.0) dT = 500.0;
         if (dT < -0.5 * T) dT = -0.5 * T;
+        const double T_was = T;
         T += dT;
-        if (fabs(dT) <= rtol * T) it_used = it + 1;
+        if (MOMENTS ? gas::newton_done<NS>(t.m.T_mid, T_was, dT, T) : fabs(dT) <= 1e-9 * T) it_used = it + 1;
     }
     return it_used;
 }
@@ -387,7 +390,7 @@ __device__ __forceinline__ void sp_local_state(SpBlock<NS> &B, const AT &A, doub
     // calculate_temp
     double Y, T;
     sp_mass_fractions(B, t, s0 / rho_loc, Y);
-    const int it = sp_T_from_u<NS, false>(B, t, Y, si_energy_mass(A.U, (float)Uint), T0_si, 1e-9, 100, on, T);
+    const int it = sp_T_from_u<NS, false, false>(B, t, Y, si_energy_mass(A.U, (float)Uint), T0_si, on, T);
     if (it < 0 && B.set == 0) atomic_status(A.status, LBMGPU_ST_NEWTON);
     T_loc = u_temp(A.U, (float)T);
 }
@@ -527,7 +530,7 @@ __device__ __forceinline__ void sp_moments(SpBlock<NS> &B, const AT &A, long n, 
     const double vol = 1.0 / (double)si_rho(A.U, (float)rho);
     const double rho_n_si = 1.0 / vol;
     double Tn;
-    const int it = sp_T_from_u<NS, fast>(B, t, Y, u_si, T_si, kNewtonTol, 100, true, Tn);
+    const int it = sp_T_from_u<NS, fast, true>(B, t, Y, u_si, T_si, true, Tn);
     const double Pn = rho_n_si * gas::kR * Tn / Wn;
     const double Tl = u_temp(A.U, (float)Tn);
     if (!valid) return;
