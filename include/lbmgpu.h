@@ -324,7 +324,9 @@ int lbmgpu_diagnostics(lbmgpu_t *h, double *out, int n_out);
  *   `epochs` passes over the samples in shuffled minibatches of `batch` (a multiple of 64)
  *   rows, the step size decaying from lr to 0 along a half cosine over the call; the
  *   standardisation and gate box are fitted on the first call or with refit; *loss = the
- *   last epoch's mean loss.
+ *   last epoch's mean loss.  Its device buffers (about 4 kB per batch row and 4 B per sample
+ *   row) stay with the handle for the next call up to 64 MiB, and are given back where a
+ *   later allocation of the handle finds no memory; larger ones are freed at the end.
  * lbmgpu_surrogate_enable: the surrogate on (after training) or off; resets the audit
  *   counters of lbmgpu_surrogate_stats.
  * lbmgpu_surrogate_eval: the network on n host rows of raw features (x: n x 12) ->

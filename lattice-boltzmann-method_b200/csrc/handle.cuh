@@ -125,9 +125,17 @@ inline int cuda_fail(cudaError_t e) {
         if (e_ != cudaSuccess) return lbmh::cuda_fail(e_); \
     } while (0)
 
+// Gives back the surrogate's training buffers, if the handle keeps any (surrogate.cu).
+bool sur_trim(lbmgpu *h);
+
 template <typename T>
 int dalloc(lbmgpu *h, T **p, size_t count) {
-    CK(cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T)));
+    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T));
+    if (e == cudaErrorMemoryAllocation && sur_trim(h)) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(reinterpret_cast<void **>(p), count * sizeof(T));
+    }
+    CK(e);
     h->bytes += count * sizeof(T);
     return 0;
 }

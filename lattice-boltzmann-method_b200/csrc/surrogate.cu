@@ -797,6 +797,11 @@ cudaError_t gemm_tn(lbmgpu *h, const __nv_bfloat16 *A, int lda, const __nv_bfloa
 // -------------------------------------------------------------------------------------
 // Host side.
 // -------------------------------------------------------------------------------------
+// Bytes of training buffers that a handle keeps after a call.  A batch of 4096 takes 18 MB; an epoch over
+// 200,000 rows takes 11.9 ms with them and 37 ms where the twenty buffers are allocated anew.  The cost
+// is that of allocating, whatever the size, so a large batch loses the least by it.
+constexpr size_t kWorkKeep = (size_t)64 << 20;
+
 struct SurState {
     // parameters: FP32 master (w), Adam moments (m, v), gradients (g), BF16 copies of the
     // weight tensors; one contiguous block each in the order w1 w2 w3 w4 b1 b2 b3 b4
@@ -824,8 +829,8 @@ struct SurState {
     bool trained = false;
     long adam_t = 0, train_steps = 0;
     double last_loss = 0.0;
-    // training buffers, kept between calls of the same batch size (freed with the handle): 4 kB per
-    // batch row and 4 B per sample row
+    // training buffers, 4 kB per batch row and 4 B per sample row, kept between calls of the same batch
+    // size up to kWorkKeep bytes; given back with the handle, or where an allocation of it finds no memory
     struct Work {
         int B = 0;
         long rows = 0, nbatch = 0;
@@ -954,6 +959,12 @@ static void work_release(lbmgpu *h, SurState &s) {
         cudaFree(p);
     h->bytes -= w.bytes;
     w = SurState::Work{};
+}
+
+bool sur_trim(lbmgpu *h) {
+    if (!h->sur || !h->sur->work.B) return false;  // none, or a call is just allocating them
+    work_release(h, *h->sur);
+    return true;
 }
 
 void sur_release(lbmgpu *h) {
@@ -1437,6 +1448,7 @@ int lbmgpu_surrogate_train(lbmgpu_t *h, int epochs, int batch, float lr, unsigne
         for (long q = 0; q < (long)nparts * bi; ++q) sum_se += parts[q];
         epoch_loss = sum_n ? sum_se / sum_n : 0.0;
     }
+    if (wk.bytes > kWorkKeep) work_release(h, s);
     if (rc) return rc;
     s.trained = true;
     s.last_loss = epoch_loss;
