@@ -140,6 +140,15 @@ int dalloc(lbmgpu *h, T **p, size_t count) {
     return 0;
 }
 
+// Frees count elements from dalloc.
+template <typename T>
+void dfree(lbmgpu *h, T *&p, size_t count) {
+    if (!p) return;
+    cudaFree(p);
+    h->bytes -= count * sizeof(T);
+    p = nullptr;
+}
+
 inline void ev_begin(lbmgpu *h, int kind, EvPair &ep, cudaStream_t st = nullptr) {
     if (!h->prof) return;
     if (h->pool.empty()) {

@@ -642,7 +642,7 @@ int lbmgpu_upload(lbmgpu_t *h, const void *mixture_aos, const void *const *speci
         for (int b = 0; b < 2; ++b) {
             if (h->bst[b]) {
                 cudaFree(h->bst[b]);
-                h->bytes -= 54 * (size_t)h->nb * sizeof(double);
+                h->bytes -= 54 * (size_t)std::max<long>(h->nb, 1) * sizeof(double);
                 h->bst[b] = nullptr;
             }
         }

@@ -1131,21 +1131,26 @@ int fit_norm(lbmgpu *h, long n) {
     return 0;
 }
 
+void free_samples(lbmgpu *h, float *&x, float *&y, uint8_t *&v, long cap) {
+    dfree(h, x, (size_t)cap * kSurIn);
+    dfree(h, y, (size_t)cap * kSurOut);
+    dfree(h, v, (size_t)cap);
+}
+
 int ensure_samples(lbmgpu *h, long cap) {
     SurState &s = *h->sur;
     if (s.ds_cap >= cap && s.ds_x) return 0;
-    cudaFree(s.ds_x);
-    cudaFree(s.ds_y);
-    cudaFree(s.ds_valid);
-    s.ds_x = s.ds_y = nullptr;
-    s.ds_valid = nullptr;
+    free_samples(h, s.ds_x, s.ds_y, s.ds_valid, s.ds_cap);
     int rc = dalloc(h, &s.ds_x, (size_t)cap * kSurIn);
     if (!rc) rc = dalloc(h, &s.ds_y, (size_t)cap * kSurOut);
     if (!rc) rc = dalloc(h, &s.ds_valid, (size_t)cap);
-    if (rc) return rc;
-    CK(cudaMemsetAsync(s.ds_valid, 0, (size_t)cap, h->stream));
-    s.ds_cap = cap;
+    s.ds_cap = rc ? 0 : cap;
     s.ds_next = 0;
+    if (rc) {
+        free_samples(h, s.ds_x, s.ds_y, s.ds_valid, cap);
+        return rc;
+    }
+    CK(cudaMemsetAsync(s.ds_valid, 0, (size_t)cap, h->stream));
     return 0;
 }
 
@@ -1160,9 +1165,7 @@ int grow_samples(lbmgpu *h, long cap) {
     if (!rc) rc = dalloc(h, &y, (size_t)cap * kSurOut);
     if (!rc) rc = dalloc(h, &v, (size_t)cap);
     if (rc) {
-        cudaFree(x);
-        cudaFree(y);
-        cudaFree(v);
+        free_samples(h, x, y, v, cap);
         return rc;
     }
     CK(cudaMemsetAsync(v, 0, (size_t)cap, h->stream));
@@ -1172,9 +1175,7 @@ int grow_samples(lbmgpu *h, long cap) {
         CK(cudaMemcpyAsync(v, s.ds_valid, (size_t)keep, cudaMemcpyDeviceToDevice, h->stream));
     }
     CK(cudaStreamSynchronize(h->stream));
-    cudaFree(s.ds_x);
-    cudaFree(s.ds_y);
-    cudaFree(s.ds_valid);
+    free_samples(h, s.ds_x, s.ds_y, s.ds_valid, s.ds_cap);
     s.ds_x = x;
     s.ds_y = y;
     s.ds_valid = v;
@@ -1259,7 +1260,7 @@ int lbmgpu_surrogate_augment(lbmgpu_t *h, long n, float span_y, float span_t, fl
                                                          n_rows, n, span_y, span_t, y_trace, seed);
     const cudaError_t e = cudaGetLastError();
     const cudaError_t e2 = cudaStreamSynchronize(h->stream);
-    cudaFree(src_d);
+    dfree(h, src_d, src.size());
     CK(e);
     CK(e2);
     s.ds_next = n_rows + n;
@@ -1491,9 +1492,9 @@ int lbmgpu_surrogate_eval(lbmgpu_t *h, const float *x, long n, float *y) {
             cudaStreamSynchronize(h->stream))
             rc = LBMGPU_E_CUDA;
     }
-    cudaFree(xd);
-    cudaFree(X);
-    cudaFree(pd);
+    dfree(h, xd, (size_t)n * kSurIn);
+    dfree(h, X, (size_t)mpad * kSurInX);
+    dfree(h, pd, (size_t)mpad * kSurOutPad);
     return rc;
 }
 
