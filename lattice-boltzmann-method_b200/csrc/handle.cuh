@@ -23,8 +23,9 @@ enum Phase { PH_BOUNDARY = 0, PH_COLLIDED = 1, PH_STREAMED = 2, PH_BC = 3, PH_SP
 // (k_mc_relax), K_STREAM_MOMENT the pull and population sums of the interior cells
 // (k_mc_gather), K_PROPS the collision parameters (k_mc_props), K_SURROGATE the chemistry
 // surrogate's features, network and integrator list, K_SOLVE the interior cells' moment
-// solve (k_mc_diffuse, k_mc_thermo), K_EFLUX the energy-flux terms of the collision (k_mc_eflux), K_CHEM
-// the stiff chemistry of every cell (k_mc_chem, ROS2 without the surrogate)
+// solve (k_mc_diffuse and k_mc_thermo: two launches a step), K_EFLUX the energy-flux terms of the
+// collision (k_mc_eflux), K_CHEM the chemistry of every cell (k_mc_chem: ROS2, or the use of the
+// surrogate's prediction; k_mc_explicit)
 enum KernelKind {
     K_COLLIDE = 0, K_STREAM_MOMENT = 1, K_OTHER = 2, K_PROPS = 3, K_SURROGATE = 4, K_SOLVE = 5, K_EFLUX = 6,
     K_CHEM = 7, K_NKINDS = 8

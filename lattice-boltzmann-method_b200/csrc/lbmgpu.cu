@@ -361,25 +361,29 @@ int launch_stream_moment(lbmgpu *h) {
     if (h->ns > 0) return lbmh::mc_launch_stream(h);
     const int c = h->cur, x = 1 - c;
     // the special cells on the side stream beside the others: disjoint cells, both read only the
-    // collision's output and the previous record
-    if (h->nb > 0) {
+    // collision's output and the previous record; in turn while kernels are timed
+    const bool beside = h->nb > 0 && !h->prof;
+    const cudaStream_t bs = beside ? h->side : h->stream;
+    if (beside) {
         CK(cudaEventRecord(h->fork, h->stream));
         CK(cudaStreamWaitEvent(h->side, h->fork, 0));
-        EvPair eb{};
-        ev_begin(h, K_OTHER, eb, h->side);
-        k_sc_special<<<(unsigned)((h->nb + kScSpBlock - 1) / kScSpBlock), kScSpBlock, 0, h->side>>>(
-            h->g, h->P, h->type, h->blist, h->pop[x], h->mom[c], h->mom[x], h->bst[c], h->bst[x], h->nb, h->status);
-        ev_end(h, eb, h->side);
-        CK(cudaGetLastError());
-        CK(cudaEventRecord(h->join, h->side));
     }
+    if (h->nb > 0) {
+        EvPair eb{};
+        ev_begin(h, K_OTHER, eb, bs);
+        k_sc_special<<<(unsigned)((h->nb + kScSpBlock - 1) / kScSpBlock), kScSpBlock, 0, bs>>>(
+            h->g, h->P, h->type, h->blist, h->pop[x], h->mom[c], h->mom[x], h->bst[c], h->bst[x], h->nb, h->status);
+        ev_end(h, eb, bs);
+        CK(cudaGetLastError());
+    }
+    if (beside) CK(cudaEventRecord(h->join, h->side));
     EvPair ep{};
     ev_begin(h, K_STREAM_MOMENT, ep);
     CK(launch_next(!h->prof && h->nb == 0, k_sc_stream_moment, grid_for(h->g.ncell), kBlock, 0, h->stream, h->g, h->P,
                    h->cflag, h->pop[x], h->mom[x], h->status));
     ev_end(h, ep);
     CK(cudaGetLastError());
-    if (h->nb > 0) CK(cudaStreamWaitEvent(h->stream, h->join, 0));
+    if (beside) CK(cudaStreamWaitEvent(h->stream, h->join, 0));
     h->cur = x;
     h->pack_mode = PK_STEPPED;
     return 0;

@@ -160,7 +160,7 @@ template <int NS, typename S>
 int explicit_step(lbmgpu *h, const lbm::McArgsT<S, double> &A, cudaStream_t st) {
     const unsigned gp = grid_for(h->g.ncell);
     EvPair ec{};
-    ev_begin(h, K_PROPS, ec, st);
+    ev_begin(h, K_CHEM, ec, st);
     bool compiled = false;
     if constexpr (NS == kin_h2_air_9::NS) {
         if (h->kin == KIN_H2_AIR_9) {

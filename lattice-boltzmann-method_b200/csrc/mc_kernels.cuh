@@ -331,8 +331,11 @@ int stream_t(lbmgpu *h) {
     EvPair es{};
     ev_begin(h, K_SOLVE, es);
     CK(launch_next(!h->prof, k_mc_diffuse<NS, S>, grid_for(h->g.ncell), kBlock, 0, h->stream, A));
-    CK(launch_next(!h->prof, k_mc_thermo<NS, S>, grid_for(h->g.ncell), kBlock, 0, h->stream, A));
     ev_end(h, es);
+    EvPair et{};
+    ev_begin(h, K_SOLVE, et);
+    CK(launch_next(!h->prof, k_mc_thermo<NS, S>, grid_for(h->g.ncell), kBlock, 0, h->stream, A));
+    ev_end(h, et);
     if (h->nb > 0) CK(cudaStreamWaitEvent(h->stream, h->join, 0));
     return 0;
 }

@@ -350,8 +350,8 @@ class Lattice:
     def kernel_times(self):
         """Per kernel kind (0 collide / population update, 1 stream+boundary+moment
         (multicomponent: the interior pull and sums), 2 other, 3 multicomponent collision
-        parameters, 4 chemistry surrogate, 5 multicomponent moment solve, 6 multicomponent
-        energy-flux terms, 7 stiff chemistry of every cell): launches and device ms."""
+        parameters, 4 chemistry surrogate, 5 multicomponent moment solve (two launches a step),
+        6 multicomponent energy-flux terms, 7 chemistry of every cell): launches and device ms."""
         launches = (ctypes.c_long * KERNEL_KINDS)()
         ms = (ctypes.c_double * KERNEL_KINDS)()
         _check(self.L.lbmgpu_kernel_times(self.h, KERNEL_KINDS, launches, ms), "lbmgpu_kernel_times")
