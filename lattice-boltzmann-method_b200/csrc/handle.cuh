@@ -186,9 +186,9 @@ inline void ev_drain(lbmgpu *h) {
 // machine's hardware threads, at most 32; ranges of at least min_items items).
 template <class F>
 void host_parallel_for(long n, const F &f, long min_items = 1024) {
-    const long hw = std::max(1L, (long)std::thread::hardware_concurrency());
-    const long nt = std::max(1L, std::min(std::min(hw, 32L), n / std::max(1L, min_items)));
-    if (nt == 1) {
+    long nt = std::min(32L, n / std::max(1L, min_items));
+    if (nt > 1) nt = std::min(nt, (long)std::thread::hardware_concurrency());
+    if (nt <= 1) {
         f(0L, n);
         return;
     }
@@ -209,6 +209,14 @@ void host_parallel_for(long n, const F &f, long min_items = 1024) {
 inline long transfer_chunk(const lbmgpu *h, long cells) {
     return std::min((long)h->stage_cells, std::max(8192L, (cells + 7) / 8));
 }
+
+// Bytes of single-component records from which host threads move them.  Below, one thread does, in one
+// chunk (downloads), and pageable records are copied from where they lie (uploads): while a bounce buffer
+// fits the caches of the cores whose threads touch it, the copy engine's accesses to its lines are slow
+// (6 MB: 650 us each way for 120 us).  By threads against not, ms: download 16^3 (6 MB) 1.02 for 0.49, 20^3
+// 1.5 for 0.84, 24^3 (18 MB) 0.85 for 1.4; upload 24^3 2.8 for 2.0, 32^3 (40 MB) 4.0 for 4.6, but 23 for 21
+// in a restart's read, whose records were just written; 40^3 (76 MB) 4.4 for 9.9 and 42 for 48.
+constexpr size_t kThreadedDownload = (size_t)16 << 20, kThreadedUpload = (size_t)64 << 20;
 
 // memcpy by host threads.
 inline void host_copy(void *dst, const void *src, size_t bytes) {

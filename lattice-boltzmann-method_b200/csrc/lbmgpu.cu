@@ -668,16 +668,16 @@ int lbmgpu_upload(lbmgpu_t *h, const void *mixture_aos, const void *const *speci
     CK(cudaMemcpyAsync(h->cflag, cf.data(), nc, cudaMemcpyHostToDevice, h->stream));
     CK(cudaMemcpyAsync(h->bid, bidh.data(), nc * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     h->cur = 0;
-    // page-locked records are copied directly; host threads fill one bounce buffer with pageable ones
+    // page-locked and few records are copied directly; host threads fill one bounce buffer with others
     // while the other's copy is under way (fork and join mark them: no step is running)
-    const bool pinned = host_pinned(host);
-    const long step = pinned ? (long)h->stage_cells : transfer_chunk(h, nc);
+    const bool direct = (size_t)nc * rs < kThreadedUpload || host_pinned(host);
+    const long step = direct ? (long)h->stage_cells : transfer_chunk(h, nc);
     const cudaEvent_t copied[2] = {h->fork, h->join};
-    if (!pinned) CK(cudaStreamSynchronize(h->stream));  // the bounce buffers' earlier copies have gone
+    if (!direct) CK(cudaStreamSynchronize(h->stream));  // the bounce buffers' earlier copies have gone
     long chunk = 0;
     for (long n0 = 0; n0 < nc; n0 += step, ++chunk) {
         const long n1 = std::min<long>(nc, n0 + step);
-        if (pinned) {
+        if (direct) {
             CK(cudaMemcpyAsync(h->stage, host + n0 * rs, (n1 - n0) * rs, cudaMemcpyHostToDevice, h->stream));
         } else {
             char *const bounce = chunk & 1 ? h->bounce2 : h->bounce;
@@ -776,8 +776,9 @@ int lbmgpu_download(lbmgpu_t *h, void *mixture_aos, void *const *species_aos) {
     const int c = h->cur;
     const long mof[6] = {h->mo.rho, h->mo.u, h->mo.v, h->mo.w, h->mo.temp, h->mo.p};
     // chunk k is packed on the device and copied into bounce buffer k % 2; while host threads merge chunk
-    // k, the device packs and copies chunk k + 1 into the other buffer
-    const long step = transfer_chunk(h, nc);
+    // k, the device packs and copies chunk k + 1 into the other buffer; few records: one chunk, one thread
+    const bool threaded = (size_t)nc * rs >= kThreadedDownload;
+    const long step = threaded ? transfer_chunk(h, nc) : (long)h->stage_cells;
     auto issue = [&](long n0, char *dst) -> int {
         const long n1 = std::min<long>(nc, n0 + step);
         CK(cudaMemsetAsync(h->stage, 0, (size_t)(n1 - n0) * rs, h->stream));  // zero padding bytes
@@ -833,9 +834,8 @@ int lbmgpu_download(lbmgpu_t *h, void *mixture_aos, void *const *species_aos) {
                     }
                 }
             }
-        });
+        }, threaded ? 1024 : n1 - n0);
     }
-    CK(cudaStreamSynchronize(h->stream));
     return LBMGPU_OK;
 }
 
