@@ -370,44 +370,47 @@ def run_reference(args, dist):
 
 
 def mc_bytes(kernel, pop_bytes, reaction=False):
-    """Algorithmic bytes per fluid cell of one multicomponent launch (9 species): every
-    population (270 planes of `pop_bytes`) read once and, by the update, written once;
-    the FP64 record and parameter planes each kernel must read or write once per cell.
+    """Algorithmic bytes per fluid cell (9 species) of the population update, and of the moments
+    as two kernels split at 91 planes of sums (per species rho_a, j_a, its P-tensor share; the
+    energy sum), for comparison with the kernels that a step launches (step_bytes):
       k_mc_relax : 270 populations in and out; per species rho_a, the 3 face terms and
                    the parameters om_a, F_a (3) [, drho_a]; shared u (3), T, rho; the
                    energy set's 7 parameters -> 9 * (4 + 4) + 5 + 7 = 84 planes [+ 9]
-      k_mc_gather, k_mc_solve : moments split at 91 planes of sums (per species rho_a, j_a, its
-                   P-tensor share; the energy sum), which the one writes and the other reads
-                   beside 21 record planes and the 36 D_ab, 88 record planes written; the
-                   device's own split is step_bytes below
-      k_mc_props : 58 record planes of the cell, 86 parameter planes written (49 + the 36
-                   D_ab + R/W) [+ HRR]
-      k_mc_eflux : 53 record planes of the cell (rho, u, T, p, rho_a, u_a, the P tensor, the
-                   heat flux) + 3 rates read, 40 read once by its neighbours, 3 written"""
+      k_mc_gather, k_mc_solve : the one writes and the other reads the sums, beside 21 record
+                   planes and the 36 D_ab, 88 record planes written"""
     if kernel == "k_mc_relax":
         return 2 * 270 * pop_bytes + (84 + (9 if reaction else 0)) * 8
-    if kernel == "k_mc_props":
-        return (58 + 86 + (1 if reaction else 0)) * 8
-    if kernel == "k_mc_eflux":
-        return (53 + 3 + 40 + 3) * 8
     if kernel == "k_mc_solve":
         return (91 + 21 + 36 + 88) * 8
     return 270 * pop_bytes + 91 * 8  # k_mc_gather
 
 
+# FP64 planes (record and collision parameters) that a step's kernels read and write, 9 species, each
+# counted once per cell whatever its neighbours read of it
+STEP_PLANES = {
+    # rho, T, p, rhoE, rho_a, u_a, X_a -> om_a, F_a (3), the 36 D_ab, omega, omega_1, theta, U, R/W
+    "k_mc_props": (4 + 9 + 27 + 9, 9 + 27 + 36 + 5),
+    # rho, u, T, p, the P tensor, the face terms Q, rho_a, u_a, omega, omega_1, R/W -> the energy flux
+    "k_mc_eflux": (6 + 6 + 3 + 9 + 27 + 3, 3),
+    # (the populations) -> rho, u, P, rhoE, rho_a, j_a
+    "k_mc_gather": (0, 4 + 6 + 1 + 9 + 27),
+    # p, X_a, the 36 D_ab, rho_a, j_a -> u_a
+    "k_mc_diffuse": (1 + 9 + 36 + 9 + 27, 27),
+    # rho, u, rhoE, T, rho_a, u_a -> T, p, X_a, the face terms Q and Q_a
+    "k_mc_thermo": (6 + 9 + 27, 2 + 9 + 3 + 27),
+    # rho, T, rho_a -> drho_a, heat release
+    "k_mc_chem": (2 + 9, 9 + 1),
+    # rho, rhoE, T, rho_a, u_a -> drho_a, heat release
+    "k_mc_explicit": (3 + 9 + 27, 9 + 1),
+}
+
+
 def step_bytes(kernel, pop_bytes, reaction=False):
-    """mc_bytes of the kernels a step launches, with the moments split where the device splits them:
-      k_mc_gather : 270 populations pulled, 47 record planes written (rho, u, P, rhoE; per
-                    species rho_a, j_a)
-      k_mc_diffuse: rho, u, T, p, rho_a, j_a and the 36 D_ab read, u_a written
-      k_mc_thermo : rho, u, rhoE, P, T, rho_a, u_a read, T, p, X_a and the 30 face terms written"""
-    if kernel == "k_mc_gather":
-        return 270 * pop_bytes + 47 * 8
-    if kernel == "k_mc_diffuse":
-        return (6 + 36 + 36 + 27) * 8
-    if kernel == "k_mc_thermo":
-        return (12 + 36 + 2 + 9 + 30) * 8
-    return mc_bytes(kernel, pop_bytes, reaction)
+    """Algorithmic bytes per fluid cell of one launch of a kernel that a step launches."""
+    if kernel == "k_mc_relax":
+        return mc_bytes(kernel, pop_bytes, reaction)
+    pops = 270 * pop_bytes if kernel == "k_mc_gather" else 0
+    return pops + 8 * sum(STEP_PLANES[kernel])
 
 
 MC_SHAPES = {"mix": "periodic", "react": "periodic", "inflow": "TYPE_I_C inflow / TYPE_O_C outflow in x, periodic y z",
@@ -631,8 +634,9 @@ def run_ours_mc(args, dist):
     lat.close()
     avg = {"k_mc_relax": kms[0] / kk, "k_mc_gather": kms[1] / kk, "k_mc_diffuse + k_mc_thermo": kms[5] / kk,
            "k_mc_props": kms[3] / kk, "k_mc_eflux": kms[6] / kk}
+    chem_kernel = "k_mc_explicit" if args.chem == "ref" else "k_mc_chem"
     if reaction and kms[7] > 0:
-        avg["k_mc_explicit" if args.chem == "ref" else "k_mc_chem"] = kms[7] / kk
+        avg[chem_kernel] = kms[7] / kk
     hbm_kernels = ("k_mc_relax", "k_mc_gather")
     dom = max(hbm_kernels, key=avg.get)  # the dominant population-moving kernel
     alg = step_bytes(dom, pop_bytes, reaction) * ncell
@@ -683,8 +687,9 @@ def run_ours_mc(args, dist):
                    "storage": ("FP32 populations (shifted), FP64 records; transport properties in FP32, the "
                                "chemistry, moment solve and temperature recovery in FP64") if pop_bytes == 4
                    else "FP64"},
-        "hbm_gbs_step": ncell * sum(step_bytes(k, pop_bytes, reaction) for k in ("k_mc_relax", "k_mc_gather", "k_mc_diffuse", "k_mc_thermo", "k_mc_props", "k_mc_eflux"))
-        / (ms / args.steps * 1e-3) / 1e9,
+        "hbm_gbs_step": ncell * sum(step_bytes(k, pop_bytes, reaction) for k in (
+            "k_mc_relax", "k_mc_gather", "k_mc_diffuse", "k_mc_thermo", "k_mc_props", "k_mc_eflux",
+            *([chem_kernel] if reaction else []))) / (ms / args.steps * 1e-3) / 1e9,
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak,
                      "traffic": ncu_traffic(dom, ncell, f"{args.workload}_{args.precision}"),
