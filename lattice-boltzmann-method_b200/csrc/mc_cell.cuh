@@ -43,11 +43,6 @@
 namespace lbm {
 
 constexpr double kSpeciesMin = 1e-8;   // SPECIES_MIN, src/headers/defines.hpp:96
-#if defined(__CUDA_ARCH__)
-constexpr bool kHostBuild = false;
-#else
-constexpr bool kHostBuild = true;
-#endif
 
 enum : int {
     RM_RHO = 0, RM_U = 1, RM_V = 2, RM_W = 3, RM_T = 4, RM_P = 5, RM_RHOE = 6, RM_P00 = 7,  // P00 P01 P02 P11 P12 P22
@@ -776,12 +771,12 @@ MC_HD void mc_chem_state(const AT &A, long n, double &rho, double *rho_a, double
 
 // The transport part of the collision parameters (lbm-collision.cpp:402-471 species rates and
 // Maxwell-Stefan force, :231-316 energy rates) in FP64 (the FP64 storage mode).  The quotients that
-// the reference rounds to float at its unit conversions stay divisions, so their floats are the
-// reference's.  The Wilke pairs multiply per-species square roots and reciprocals on the device
-// (45 pairs: 18 square roots and reciprocals in place of 225; rounding-level differences, as its exp
-// and log make them anyway); the host build, which restates the reference operation by operation,
-// keeps the quotients.  Every loop is unrolled: the arrays live in registers.
-template <int NS, class AT>
+// the reference rounds to float at its unit conversions are divisions, so their floats are the
+// reference's.  EXACT: every other quotient too, operation by operation the reference's (the host
+// build's steps).  The device instead multiplies per-species square roots and reciprocals in the Wilke
+// pairs (45 pairs: 18 square roots and reciprocals in place of 225), forms a pair's force coefficient
+// once and one reciprocal per species for the force; within 1e-12 of the exact form.
+template <int NS, bool EXACT, class AT>
 MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a, const double *Y, const double *X,
                              double W, double T_si, double P_si, double Uint) {
     const gas::Tables &t = *A.tab;
@@ -815,7 +810,7 @@ MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a,
 #pragma unroll
             for (int b = a; b < NS; ++b) {
                 double pab, pba;
-                if (kHostBuild) {
+                if (EXACT) {
                     const double f1 = 1.0 + sqrt(mu_k[a] / mu_k[b]) * t.sqrt4W[a][b];
                     pab = f1 * f1 / t.wilke_den[a][b];
                     pba = mu_k[b] / mu_k[a] * t.m.W[a] / t.m.W[b] * pab;
@@ -890,9 +885,9 @@ MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a,
 #pragma unroll
         for (int b = 0; b < a; ++b) {
             const double D = Pr[(long)pr_d<NS>(a, b) * A.ncell + n];
-            // the reference's -p X_a X_b / D_ab, per ordered pair in the host build
+            // the reference's -p X_a X_b / D_ab
             const double kab = -1.0 * p * Xs[a] * Xs[b] / D;
-            const double kba = kHostBuild ? -1.0 * p * Xs[b] * Xs[a] / D : kab;
+            const double kba = EXACT ? -1.0 * p * Xs[b] * Xs[a] / D : kab;
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 const double du = ua[a][d] - ua[b][d];
@@ -904,7 +899,7 @@ MC_HDN void mc_transport_f64(const AT &A, long n, double p, const double *rho_a,
     for (int a = 0; a < NS; ++a) {
         const double s = dt / rho_a[a];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) prp(pr_f<NS>(a, d), kHostBuild ? F[a][d] * dt / rho_a[a] : F[a][d] * s);
+        for (int d = 0; d < 3; ++d) prp(pr_f<NS>(a, d), EXACT ? F[a][d] * dt / rho_a[a] : F[a][d] * s);
     }
 }
 
@@ -1092,8 +1087,8 @@ MC_HDN void mc_chem_explicit(const AT &A, long n, const Net &net) {
 }
 
 // The collision parameters of one cell.  CHEM: the chemistry to run with it (the host build; the
-// device runs the chemistry in kernels of its own, CHEM_OFF here).
-template <int NS, int CHEM, class AT>
+// device runs the chemistry in kernels of its own, CHEM_OFF here).  EXACT: see mc_transport_f64.
+template <int NS, int CHEM, bool EXACT = true, class AT>
 MC_HDN void mc_props_cell(const AT &A, long n) {
     const gas::Tables &t = *A.tab;
     const typename AT::R *Rc = A.rec_cur;
@@ -1118,7 +1113,7 @@ MC_HDN void mc_props_cell(const AT &A, long n) {
     if constexpr (sizeof(typename AT::P) == sizeof(float))
         mc_transport_f32<NS>(A, n, p, rho_a, Y, X, W, T_si, P_si, Uint);
     else
-        mc_transport_f64<NS>(A, n, p, rho_a, Y, X, W, T_si, P_si, Uint);
+        mc_transport_f64<NS, EXACT>(A, n, p, rho_a, Y, X, W, T_si, P_si, Uint);
 }
 
 // The energy-flux terms of the energy collision (lbm-collision.cpp:265-316): the enthalpy

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_mc_props(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;
     lbmh::step_begin();
     if (n >= A.ncell || !(A.cflag[n] & CF_FLUID)) return;
-    mc_props_cell<NS, CHEM_OFF>(A, n);
+    mc_props_cell<NS, CHEM_OFF, false>(A, n);
 }
 
 template <int NS, typename S>
