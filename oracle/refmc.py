@@ -33,9 +33,15 @@ def available(reaction=False, fast=False):
     return os.path.exists(_path(reaction, fast))
 
 
+class ReferenceMissing(OSError):
+    """The library was not built: it needs the reference's sources (oracle/Makefile)."""
+
+
 def lib(reaction=False, fast=False):
     key = (reaction, fast)
     if key not in _libs:
+        if not available(reaction, fast):
+            raise ReferenceMissing(f"reference library not built here: {os.path.basename(_path(reaction, fast))}")
         L = ctypes.CDLL(_path(reaction, fast))
         vp = ctypes.c_void_p
         L.ref_mc_set_mech.argtypes = [vp]
