@@ -56,7 +56,7 @@ struct SpOff {
 struct lbmgpu {
     lbmgpu_desc d{};
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;           // multicomponent: the boundary cells beside the interior
+    cudaStream_t side = nullptr;  // the boundary cells beside the interior, the chemistry beside the transport
     cudaEvent_t fork = nullptr, join = nullptr;
     lbm::ScGeom g{};
     lbm::ScPhys P{};

@@ -4,8 +4,8 @@
 // Reference path replaced (farrasarira/Lattice-Boltzmann-Method, single component):
 //   LBM::Collide            src/lbm-collision.cpp:9-99     -> k_sc_collide
 //   LBM::Streaming          src/lbm-streaming.cpp:3-119    -> k_sc_stream_moment (pull)
-//   LBM::TMS_BC             src/lbm-bc.cpp:341-460, 809-938, 1111-1229 -> k_sc_stream_moment
-//   LBM::calculate_moment   src/lbm-moment.cpp:11-125      -> k_sc_stream_moment
+//   LBM::TMS_BC             src/lbm-bc.cpp:341-460, 809-938, 1111-1229 -> k_sc_special
+//   LBM::calculate_moment   src/lbm-moment.cpp:11-125      -> k_sc_stream_moment, k_sc_special
 //   LBM::Init               src/lbm-init.cpp:8-82          -> k_sc_init
 #include <cuda_runtime.h>
 

@@ -35,10 +35,11 @@ using namespace lbmh;
 
 // Transport part of the collision parameters of every fluid cell (the chemistry runs in kernels of
 // its own, mc_chem.cuh), one thread per cell.  Bound by the latency of its FP64 chains and of the record
-// loads, not by HBM; three blocks per SM (168 registers), the species loops unrolled, so the
-// per-species arrays live in registers, the species velocities loaded where the Maxwell-Stefan force
-// uses them.  FP64 storage, 48 x 40 x 37 cells: 189 us with rolled loops (920 B of local arrays) and
-// 400 divisions per cell, 119 us now; FP32 storage, 96^3: 523 -> 502 us.
+// loads, not by HBM; three blocks per SM (168 registers), the species loops unrolled, so that no
+// per-species array is indexed in local memory (nine species, FP64: 184 B of spills; FP32: 8 B), the
+// species velocities loaded where the Maxwell-Stefan force uses them.  FP64 storage, 48 x 40 x 37 cells:
+// 189 us with rolled loops (920 B of local arrays) and 400 divisions per cell, 119 us unrolled, 110 us
+// with the diffusion coefficients' pairs rolled again (mc_transport_f64); FP32 storage, 96^3: 523 -> 502 us.
 template <int NS, typename S>
 __global__ void __launch_bounds__(kBlock, 3) k_mc_props(McArgsT<S, double> A) {
     const long n = (long)blockIdx.x * blockDim.x + threadIdx.x;

@@ -10,7 +10,8 @@
 // The planes between them are the record's own (the gather wrote 91 planes of sums for the solve to
 // read back; memory per cell 728 B less).  One kernel for the last two held the 9 x 9 factor and the
 // temperature iteration in one thread: 255 registers, eight warps per SM, a third of the time waiting
-// for memory; now three and five blocks of 128 threads per SM (168 and 96 registers).  All of a
+// for memory; now three and five blocks of 128 threads per SM (168 and 96 registers; nine species spill
+// 168 B in FP64 and 88 B in FP32, and 72 B).  All of a
 // thread's loads are issued before its cell's flag is known.
 // Measured, 96^3 FP32 storage: gather 387 -> 281 us (1456 B a cell: 4.6 TB/s), solve 456 -> 344 us;
 // 48 x 40 x 37 FP64: 45 -> 44 and 108 -> 73 us.  The diffusion kernel at two blocks per SM (198

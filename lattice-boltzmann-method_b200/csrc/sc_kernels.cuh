@@ -97,11 +97,12 @@ __device__ __forceinline__ int pull_at(const PullSrc &s, int l) {
     return s.X[cidx(cx(l))] + s.Y[cidx(cy(l))] + s.Z[cidx(cz(l))];
 }
 
-// The per-axis factors with u_a^2 rounded by itself before theta is added, for the axes from FIRST on (a
-// product with one use only would be fused into the sum).  Both population sets, in their own threads, and
-// the steps after an upload and later ones then round as they did in one thread per cell, to the bit: a
-// velocity component that decays to 1e-7 of the sound speed keeps only nine digits through any other
-// rounding.
+// The per-axis factors with u_a^2 rounded by itself before theta is added, for the axes from FIRST on; the
+// axes before are left to the compiler, which fuses a product with one use only into the sum.  With
+// CUDA 12.9 both population sets, in their own threads, and the steps after an upload and later ones then
+// round as they did in one thread per cell, to the bit; another compiler's choice, or one rounding for all
+// axes, is as good a rounding (1e-12 of each field's scale), but a velocity component that has
+// decayed to 1e-7 of the sound speed moves by 1e-9 of itself with it.
 template <int FIRST>
 __device__ __forceinline__ void axis_feq_sc(AxisF<double> &F, const double u[3], double theta, const double corr[3]) {
 #pragma unroll
