@@ -1228,7 +1228,7 @@ def run_ours_turb(args, dist):
         "config": {"workload": turb_name(args, N), "cells": ncell,
                    "parallelism": (f"x-slabs{dist.world} (one {N}^3 box per GPU, halos over NCCL)" if dist.world > 1
                                    else ("x-slab loopback check" if slabs else "single GPU")),
-                   "l2": "state larger than L2 (86 GB at 258^3 FP32), no flush",
+                   "l2": "state larger than L2 (74 GB at 258^3 FP32), no flush",
                    "storage": ("FP32 populations (shifted), FP64 records; transport properties in FP32, the "
                                "chemistry, moment solve and temperature recovery in FP64") if pop_bytes == 4
                    else "FP64"},

@@ -16,8 +16,8 @@
 //
 // Measured (B200, time of the kernel beside the interior's gather and solve): 8,256 cells of the
 // 512 x 8 x 8 flame channel, FP32 storage, 436 -> 149 us (the step 785 -> 491 us); 3,840 cells of a
-// 64 x 48 x 40 inflow layer, FP64, 494 -> 132 us (1041 -> 823 us).  What is left is instruction
-// fetch and the fixed latencies of one pass through the code by ten warps per SM; one copy of each
+// 64 x 48 x 40 inflow layer, FP64, 494 -> 132 us (1041 -> 823 us); alone 110 and 62 us.  What is left is
+// instruction fetch and the fixed latencies of one pass through the code by ten warps per SM; one copy of each
 // part of the passes (the loops over pass and stage below) took 231 to 180 us.  The populations in
 // shared memory with two blocks per SM (96 registers) was no faster (182 us there, 160 us for the
 // inflow layer).
