@@ -198,7 +198,9 @@ __device__ __forceinline__ void relax_energy_dev(const AT &A, long n, bool in, c
     AxisG<double> G;
     axis_geq(G, Ui, theta, um);
     P *const dst = A.pop_dst + (long)27 * NS * nc;
-    const double kq = 0.5 * (om1 - om);
+    // the flux correction acts along the six axes; a value of it that is not finite reaches what the products
+    // with zero reach in the reference: the other axes (z), and every direction (kq in omn)
+    const double kq = 0.5 * (om1 - om), z = 0.0 * dq[0] + 0.0 * dq[1] + 0.0 * dq[2], omn = om1 + 0.0 * kq;
 #pragma unroll
     for (int ix = 0; ix < 3; ++ix) {
         const double px = rho * G.P[0][ix], tx = rho * (G.E * G.P[0][ix] + G.A[0][ix]);
@@ -209,9 +211,8 @@ __device__ __forceinline__ void relax_energy_dev(const AT &A, long n, bool in, c
             for (int iz = 0; iz < 3; ++iz) {
                 const int l = dir3(ix, iy, iz);
                 const double g = (double)v[l], gq = B * G.P[2][iz] + C * G.A[2][iz];
-                double out = g + om1 * ((shifted ? gq - sh[l] : gq) - g);
-                if (csq(l) == 1)  // the flux correction acts along the six axes
-                    out += kq * (cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2]));
+                double out = g + omn * ((shifted ? gq - sh[l] : gq) - g);
+                if (csq(l) == 1) out += kq * ((cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2])) + z);
                 dst[(long)l * nc + n] = (P)out;
             }
         }
