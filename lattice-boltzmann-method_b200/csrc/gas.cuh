@@ -555,8 +555,10 @@ GAS_HD void net_production(const Tables &t, double T, const double *C, double *w
 // net_production for NS species known at compile time: each reaction's factors formed where it is
 // evaluated, its products and sums over the dense stoichiometry tables, so that every array is
 // indexed by compile-time constants; the products run in species order instead of the order
-// the reaction lists its species, which moves results by rounding only.  gRT: g_k/RT at T.
-template <int NS>
+// the reaction lists its species, which moves results by rounding only.  gRT: g_k/RT at T.  LISTED: a
+// reaction adds to the species it produces or consumes only, so that a rate that is not finite leaves the
+// others' as the reference does.
+template <int NS, bool LISTED = false>
 GAS_HD void net_production_dense(const Tables &t, double T, double logT, double invT, double invRT, double log_cref,
                                  const double *gRT, const double *C, double *w) {
     const lbmgpu_mech &m = t.m;
@@ -602,7 +604,8 @@ GAS_HD void net_production_dense(const Tables &t, double T, double logT, double 
         }
         const double q = fwd - rev;
 #pragma unroll
-        for (int k = 0; k < NS; ++k) w[k] += t.nu_net[r][k] * q;
+        for (int k = 0; k < NS; ++k)
+            if (!LISTED || t.nu_net[r][k] != 0.0) w[k] += t.nu_net[r][k] * q;
     }
 }
 
@@ -619,7 +622,7 @@ struct DenseNet {
             const double *a = nasa(t, k, T);
             gRT[k] = h_RT_q(t, k, T) - (a[0] * logT + T * (a[1] + T * (a[2] / 2 + T * (a[3] / 3 + T * a[4] / 4))) + a[6]);
         }
-        net_production_dense<NS>(t, T, logT, 1.0 / T, 1.0 / (kR * T), log(kOneAtm / (kR * T)), gRT, C, w);
+        net_production_dense<NS, true>(t, T, logT, 1.0 / T, 1.0 / (kR * T), log(kOneAtm / (kR * T)), gRT, C, w);
     }
 };
 struct TableNet {

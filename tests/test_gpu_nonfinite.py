@@ -51,14 +51,16 @@ def hostlib(tmp_path_factory):
 
 @pytest.mark.parametrize("steps", [1, 2, 3])
 @pytest.mark.parametrize("field,value", BAD[:2])
-@pytest.mark.parametrize("walls", [False, True])
-def test_multicomponent(hostlib, walls, field, value, steps):
-    m = mech.h2_air_9()
-    mix, sp = W.flame_channel_mc(m, 11, 8, 7) if walls else W.mixing_layer_mc(m, 9)
+@pytest.mark.parametrize("name,walls,chem", [("h2_air_9", False, 0), ("h2_air_9", True, 0), ("h2_air_9", False, 1),
+                                             ("ch4_2s", False, 1), ("c3h8_2s", False, 1)])
+def test_multicomponent(hostlib, name, walls, chem, field, value, steps):
+    m = getattr(mech, name)()
+    fuel = {"h2_air_9": "H2", "ch4_2s": "CH4", "c3h8_2s": "C3H8"}[name]
+    mix, sp = W.flame_channel_mc(m, 11, 8, 7) if walls else W.mixing_layer_mc(m, 9, T_hi=1500.0, fuel=fuel)
     mix[field][4, 4, 4] = value
     fl = (mix["type"] == W.TYPE_F).reshape(-1)
-    want, st, pops = host_run(hostlib, m, mix, sp, 0, steps, pops=True)
-    with lbmgpu.Lattice(*mix.shape, mech=m, dtype=W.MIXTURE_MC, species_dtype=W.SPECIES, dx_dt=W.FLAME_UNITS,
+    want, st, pops = host_run(hostlib, m, mix, sp, chem, steps, pops=True)
+    with lbmgpu.Lattice(*mix.shape, mech=m, dtype=W.MIXTURE_MC, species_dtype=W.SPECIES, dx_dt=W.FLAME_UNITS, chem=chem,
                         library=lbmgpu.NOFMA_LIB_PATH) as lat:
         lat.upload(mix, sp)
         lat.init()
