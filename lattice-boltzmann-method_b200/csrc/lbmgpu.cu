@@ -129,15 +129,17 @@ __global__ void __launch_bounds__(2 * kBlock, 2)
     for (int a = 0; a < 3; ++a) dq[a] = S[a] + 0.5 * dt * vel[a] * dQ[a];
     AxisG<double> G;
     axis_geq_sc<LOCAL ? 0 : 1>(G, Uint, theta, vel);
-    // the flux correction acts along the six axes; a value of it that is not finite reaches what the products
-    // with zero reach in the reference: the other axes (z), and every direction (omn)
-    const double z = 0.0 * dq[0] + 0.0 * dq[1] + 0.0 * dq[2], omn = om1 + 0.0 * (om - om1);
+    // the flux correction acts along the six axes; a component that is not finite reaches the other axes too,
+    // through the reference's products with zero
+    const double z = 0.0 * dq[0] + 0.0 * dq[1] + 0.0 * dq[2];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) dq[a] += z;
 #pragma unroll
     for (int l = 0; l < 27; ++l) {
         const double gq = __dmul_rn(rho, geq_l(l, 1.0, G));
-        double out = v[l] + omn * (gq - v[l]);
+        double out = v[l] + om1 * (gq - v[l]);
         if (csq(l) == 1) {
-            const double gs = gq + 0.5 * ((cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2])) + z);
+            const double gs = gq + 0.5 * (cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2]));
             out += (om - om1) * (gq - gs);
         }
         d0[(long)l * nc] = out;

@@ -199,8 +199,8 @@ __device__ __forceinline__ void relax_energy_dev(const AT &A, long n, bool in, c
     axis_geq(G, Ui, theta, um);
     P *const dst = A.pop_dst + (long)27 * NS * nc;
     // the flux correction acts along the six axes; a value of it that is not finite reaches what the products
-    // with zero reach in the reference: the other axes (z), and every direction (kq in omn)
-    const double kq = 0.5 * (om1 - om), z = 0.0 * dq[0] + 0.0 * dq[1] + 0.0 * dq[2], omn = om1 + 0.0 * kq;
+    // with zero reach in the reference: the other axes (kq), and every direction (omn)
+    const double omn = om1 + 0.0 * (om1 - om), kq = 0.5 * (om1 - om) + 0.0 * dq[0] + 0.0 * dq[1] + 0.0 * dq[2];
 #pragma unroll
     for (int ix = 0; ix < 3; ++ix) {
         const double px = rho * G.P[0][ix], tx = rho * (G.E * G.P[0][ix] + G.A[0][ix]);
@@ -212,7 +212,7 @@ __device__ __forceinline__ void relax_energy_dev(const AT &A, long n, bool in, c
                 const int l = dir3(ix, iy, iz);
                 const double g = (double)v[l], gq = B * G.P[2][iz] + C * G.A[2][iz];
                 double out = g + omn * ((shifted ? gq - sh[l] : gq) - g);
-                if (csq(l) == 1) out += kq * ((cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2])) + z);
+                if (csq(l) == 1) out += kq * (cx(l) ? cx(l) * dq[0] : (cy(l) ? cy(l) * dq[1] : cz(l) * dq[2]));
                 dst[(long)l * nc + n] = (P)out;
             }
         }
